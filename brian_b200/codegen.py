@@ -107,8 +107,8 @@ class _Emitter(object):
             if op == "/" and self.fast is not None:
                 k = self.fast.slot(node.right)
                 if k is not None:
-                    return "bg_div_fast(%s, %s, bg_y%d, bg_t%d, suspect)" % (
-                        self.expr(node.left), self.expr(node.right), k, k)
+                    return "bg_div_fast(%s, %s, bg_r%d, bg_seen)" % (
+                        self.expr(node.left), self.expr(node.right), k)
             return "(%s %s %s)" % (self.expr(node.left), op, self.expr(node.right))
         if isinstance(node, ast.Call):
             if not isinstance(node.func, ast.Name) or node.func.id not in _FUNCS1 or len(node.args) != 1 \
@@ -164,11 +164,11 @@ def _cname(name):
 class _FastDivisions(object):
     """Divisions whose divisor depends only on parameters the reset never
     assigns (and on constants) divide by a per-simulation reciprocal fixed at
-    load time.  Each gets members bg_y<k> (the reciprocal, double) and
-    bg_t<k> (the dividend magnitude below which the fast form may round
-    differently, or a guard exponent for double).  The kernel checks those
-    conditions branch-free and redoes a block with IEEE division when any
-    dividend falls outside them, so results equal plain division."""
+    load time.  Each gets a member bg_r<k> (the reciprocal), and the model's
+    bg_lo and bg_hi the range of dividends for which every fast form rounds
+    like IEEE division.  The kernel collects the dividends' range branch-free
+    (bg_seen) and redoes a block with IEEE division when one fell outside, so
+    results equal plain division."""
 
     def __init__(self, base, invariant):
         self.base = base            # emitter over the load-time names
@@ -193,26 +193,14 @@ class _FastDivisions(object):
         return self.keys.index(key)
 
     def declarations(self):
-        sc = self.base.scalar
-        return "".join("    double bg_y%d;\n    %s bg_t%d;\n" % (k, sc, k) for k in range(len(self.keys)))
+        return "".join("    BgRcp<scalar> bg_r%d;\n" % k for k in range(len(self.keys)))
 
     def setup(self):
-        """Reciprocal and dividend bound of each divisor; a divisor outside
+        """Reciprocal and dividend range of each divisor; a divisor outside
         the range where the fast forms are exact (zero, subnormal, huge,
         infinite, NaN) sends the whole simulation down the IEEE path
         (bg_exact)."""
-        out = []
-        for k, key in enumerate(self.keys):
-            if self.base.scalar == "float":
-                out.append("{ const float b = %s; bg_y%d = 1.0 / (double)b; "
-                           "if (!(fabsf(b) >= 0x1p-126f && fabsf(b) <= 0x1p+126f)) bg_exact = true; "
-                           "bg_t%d = (float)(0x1p-126 * fmax(1.0, fabs((double)b)) * (1.0 + 0x1p-20)); }"
-                           % (key, k, k))
-            else:
-                out.append("{ const double b = %s; bg_y%d = 1.0 / b; "
-                           "if (!(fabs(b) >= 0x1p-100 && fabs(b) <= 0x1p+100)) bg_exact = true; "
-                           "bg_t%d = 0x1p-900; }" % (key, k, k))
-        return "\n".join(out)
+        return "\n".join("bg_rcp_set(bg_r%d, %s, bg_lo, bg_hi, bg_exact);" % (k, key) for k, key in enumerate(self.keys))
 
 
 class ModelCode(object):

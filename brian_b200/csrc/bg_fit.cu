@@ -43,6 +43,7 @@ int fail(int code, const std::string &m) { return bg_internal_fail(code, m.c_str
 
 constexpr int kSimThreads = 128;    // must match __launch_bounds__ in the template
 constexpr int kAuxThreads = 256;
+constexpr int kQueueInts = 64 + 256;   // BG_CLASSES + BG_SM_SLOTS of the template
 
 // Host image of the template's FitArgs (same field order and types).
 struct FitArgsHost {
@@ -62,9 +63,9 @@ struct FitArgsHost {
     const int *order;
     int *rec;
     int *rec_n;
-    int *next_task;
+    int *queue;
     long long ns;
-    int Tstart, Tend, onset, rec_cap;
+    int Tstart, Tend, onset, rec_cap, nsm;
 };
 
 std::vector<std::string> split_names(const char *names) {
@@ -115,15 +116,16 @@ int assemble_source(int precision, const bg_fit_model *model, double dt, int del
       << kFitHelperSource
       << "struct Model {\n";
     for (auto &n : names) o << "    scalar s_" << n << ";\n";
-    o << "    bool bg_exact;\n" << nz(model->aux_decl) << "\n";
+    o << "    bool bg_exact;\n    scalar bg_lo, bg_hi;\n" << nz(model->aux_decl) << "\n";
     o << "    __device__ __forceinline__ void load(const scalar *S, long long ns, long long i) {\n";
     for (size_t k = 0; k < names.size(); ++k) o << "        s_" << names[k] << " = S[" << k << "LL * ns + i];\n";
-    o << "        bg_exact = false;\n" << nz(model->setup_code) << "\n";
+    o << "        bg_exact = false;\n        bg_lo = 0;\n        bg_hi = " << (precision == 32 ? "__int_as_float(0x7f800000)" : "__longlong_as_double(0x7ff0000000000000LL)") << ";\n" << nz(model->setup_code) << "\n";
     o << "    }\n    __device__ __forceinline__ void store(scalar *S, long long ns, long long i) const {\n";
     for (size_t k = 0; k < names.size(); ++k) o << "        S[" << k << "LL * ns + i] = s_" << names[k] << ";\n";
     o << "    }\n    __device__ __forceinline__ void update(const scalar I_in, const scalar t) {\n"
       << nz(model->update_code) << "\n    }\n"
-      << "    __device__ __forceinline__ void update_fast(const scalar I_in, const scalar t, bool &suspect) {\n"
+      << "    template <class SEEN>\n    __device__ __forceinline__ void update_fast(const scalar I_in, const scalar t, "
+         "bool &suspect, SEEN &bg_seen) {\n"
       << (has_fast ? nz(model->update_fast_code) : "update(I_in, t);") << "\n    }\n"
       << "    __device__ __forceinline__ bool threshold(const scalar I_in, const scalar t) const {\n"
       << "        return " << (model->threshold_code && *model->threshold_code ? model->threshold_code : "false")
@@ -211,7 +213,7 @@ struct bg_fit {
     int rec_cap = 0;
     int onset = 0;
     int max_steps = 0;
-    int *next_task = nullptr;
+    int *queue = nullptr;
     int nsm = 148;
     int blocks_per_sm = 2;      // resident simulation blocks per SM (bg_fit_autotune)
     // gamma
@@ -484,18 +486,21 @@ int sim_launch(bg_fit *h, int Tstart, int Tend) {
     a.order = h->order;
     a.rec = h->rec_cap > 0 ? h->rec : nullptr;
     a.rec_n = h->rec_cap > 0 ? h->rec_n : nullptr;
-    a.next_task = h->next_task;
+    a.queue = h->queue;
+    a.nsm = h->nsm;
     a.ns = h->ns;
     a.Tstart = Tstart;
     a.Tend = Tend;
     a.onset = h->onset;
     a.rec_cap = h->rec_cap;
     void *args[] = {&a};
-    // persistent warps pulling 32-simulation tasks; no more blocks than tasks
+    // persistent warps pulling 32-simulation tasks; with few tasks, one a block
+    // (a task's warp runs alone on its SM: four of them on one SM's
+    // schedulers share its issue slots and L1)
     const long long ntasks = (h->ns + 31) / 32;
     const long long want = (long long)h->nsm * h->blocks_per_sm;
-    const unsigned grid = (unsigned)std::max(1LL, std::min(want, (ntasks + kSimThreads / 32 - 1) / (kSimThreads / 32)));
-    FCK(cudaMemsetAsync(h->next_task, 0, sizeof(int), h->stream));
+    const unsigned grid = (unsigned)std::max(1LL, std::min(want, ntasks));
+    FCK(cudaMemsetAsync(h->queue, 0, kQueueInts * sizeof(int), h->stream));
     FCK(cudaLaunchKernel((const void *)h->kern, dim3(grid), dim3(kSimThreads), args, 0, h->stream));
     ++h->sim_launches;
     return BG_OK;
@@ -595,7 +600,7 @@ BG_API int bg_fit_create(bg_fit **out, int device, int precision, const bg_fit_m
     cudaError_t e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaLibraryLoadData(&h->lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
     if (e == cudaSuccess) e = cudaLibraryGetKernel(&h->kern, h->lib, "bg_fit_sim");
-    if (e == cudaSuccess) e = cudaMalloc((void **)&h->next_task, sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&h->queue, kQueueInts * sizeof(int));
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->nsm, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
@@ -618,7 +623,7 @@ BG_API int bg_fit_destroy(bg_fit *h) {
     free_ptr(h->nspikes); free_ptr(h->order); free_ptr(h->flags); free_ptr(h->rec); free_ptr(h->rec_n);
     free_ptr(h->tlen); free_ptr(h->trate); free_ptr(h->fit); free_ptr(h->dimvar); free_ptr(h->X); free_ptr(h->V);
     free_ptr(h->Xl); free_ptr(h->lfit); free_ptr(h->Xg); free_ptr(h->gfit); free_ptr(h->lo); free_ptr(h->hi);
-    free_ptr(h->next_task);
+    free_ptr(h->queue);
     if (h->lib) cudaLibraryUnload(h->lib);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
