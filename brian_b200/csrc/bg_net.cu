@@ -19,6 +19,7 @@
 
 #include "bg_kernels.cuh"
 #include "bg_persist.cuh"
+#include "bg_cluster_host.h"
 #include "bg_synpersist.cuh"
 #include "bg_batch.cuh"
 #include "bg_rtc.h"
@@ -65,6 +66,7 @@ struct HGroup {
     std::vector<std::string> gen_names;
     std::string gen_update, gen_threshold, gen_reset;
     cudaLibrary_t gen_lib = nullptr; cudaKernel_t gen_kernel = nullptr;
+    cudaLibrary_t gen_clib = nullptr; cudaKernel_t gen_ckernel = nullptr;   // the cluster kernel around the model
     bool generated() const { return !gen_update.empty() || !gen_threshold.empty() || !gen_reset.empty(); }
 };
 // A std::vector that leaves new elements uninitialised: the large host
@@ -128,6 +130,7 @@ struct HConn {
     // rows and the table {0, w} (not part of the saved state: every launch
     // ends with the ring delivered)
     uint16_t *dDirRing = nullptr; void *dDirTable = nullptr; int dir_md = 0;
+    int64_t dir_kmax = -1;             //   its largest in-degree (-1: not counted)
     int64_t *dColptr = nullptr, *dColk = nullptr; int32_t *dColsrc = nullptr;
     int64_t wcount() const { return dense ? sn * tn : nnz; }
 };
@@ -216,6 +219,12 @@ struct bg_net {
     // persistent single-launch path (see bg_persist.cuh); empty when the
     // network does not have its shape
     std::function<cudaError_t(cudaStream_t, int nsteps)> persist;
+    // the cluster kernel's shape (bg_cluster.cuh), npt 0 when the network does not have it
+    struct ClusterPlan {
+        int npt = 0, blocks = 0, rows[2] = {0, 0}, off_ring[2] = {0, 0}, off_rows[2] = {0, 0}, off_syn[2] = {-1, -1}, off_tab[2] = {-1, -1},
+            off_rec = 0;
+        size_t smem = 0;
+    } cluster;
     unsigned int *dArrived = nullptr;
     int *dUsePull3 = nullptr;           // Synapses persistent kernel: overflow flags by step mod 3
     int *dPBinCnt = nullptr; unsigned long long *dPBinKey = nullptr; double *dPBinT = nullptr;   //   and its bins
@@ -266,12 +275,9 @@ cudaError_t launch_head(const bg::HeadArgs<T> &a, int nvar, int64_t blocks, cuda
     }
 }
 
-// The head kernel of a group with a generated model: the engine's kernel
-// sources with a model policy over the group's registers (head_body).
-template <typename T>
-int compile_generated_head(HGroup &g) {
-    if (g.gen_kernel) return BG_OK;
-    const char *sc = sizeof(T) == 8 ? "double" : "float";
+// The engine's kernel sources with a group's generated model as a policy over
+// its registers (GenModel).
+std::string generated_source(const HGroup &g) {
     std::string src = "#define BG_GENERATED_MODEL 1\n";
     for (const char *const *p = kNetRtcSource; *p; ++p) src += *p;
     auto load = [&](bool cnst) {
@@ -303,16 +309,44 @@ int compile_generated_head(HGroup &g) {
            "        (void)t; (void)I_in; (void)reset_on;\n" +
            load(false) + g.gen_reset + "\n" + store() + "    }\n";
     src += "};\n}  // namespace bg\n";
-    src += std::string("extern \"C\" __global__ void __launch_bounds__(bg::kHeadThreads, 2) bg_gen_head(const bg::HeadArgs<") +
-           sc + "> a) {\n    bg::head_body<" + sc + ", " + std::to_string(std::max(1, g.nvar)) + ", bg::GenModel>(a);\n}\n";
+    return src;
+}
+
+int compile_generated(const std::string &src, const char *name, cudaLibrary_t *lib, cudaKernel_t *kernel) {
     std::vector<char> cubin;
     std::string log;
     int rc = bg_nvrtc_compile(src, &cubin, &log);
     if (rc) return rc;
-    cudaError_t e = cudaLibraryLoadData(&g.gen_lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
-    if (e == cudaSuccess) e = cudaLibraryGetKernel(&g.gen_kernel, g.gen_lib, "bg_gen_head");
+    cudaError_t e = cudaLibraryLoadData(lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0);
+    if (e == cudaSuccess) e = cudaLibraryGetKernel(kernel, *lib, name);
     if (e != cudaSuccess) return fail(BG_ECUDA, std::string("generated group kernel: ") + cudaGetErrorString(e));
     return BG_OK;
+}
+
+// The head kernel of a group with a generated model (head_body).
+template <typename T>
+int compile_generated_head(HGroup &g) {
+    if (g.gen_kernel) return BG_OK;
+    const std::string sc = sizeof(T) == 8 ? "double" : "float";
+    return compile_generated(generated_source(g) +
+                                 "extern \"C\" __global__ void __launch_bounds__(bg::kHeadThreads, 2) bg_gen_head(const bg::HeadArgs<" +
+                                 sc + "> a) {\n    bg::head_body<" + sc + ", " + std::to_string(std::max(1, g.nvar)) +
+                                 ", bg::GenModel>(a);\n}\n",
+                             "bg_gen_head", &g.gen_lib, &g.gen_kernel);
+}
+
+// The cluster kernel of a network of one such group (cluster_body).
+template <typename T>
+int compile_generated_cluster(HGroup &g, int npt, bool multi, int pat) {
+    if (g.gen_ckernel) return BG_OK;
+    const std::string sc = sizeof(T) == 8 ? "double" : "float";
+    return compile_generated(generated_source(g) +
+                                 "extern \"C\" __global__ void __launch_bounds__(" + (multi ? "bg::kClusterThreads + 32" : "bg::kClusterThreads") +
+                                 ", 1) bg_gen_cluster(const "
+                                 "__grid_constant__ bg::ClusterArgs<" + sc + "> a) {\n    bg::cluster_body<" + sc + ", " +
+                                 std::to_string(std::max(1, g.nvar)) + ", " + std::to_string(npt) +
+                                 (multi ? ", false, true, " : ", false, false, ") + std::to_string(pat) + ", bg::GenModel>(a);\n}\n",
+                             "bg_gen_cluster", &g.gen_clib, &g.gen_ckernel);
 }
 
 template <typename T>
@@ -377,7 +411,8 @@ int build_group(bg_net *net, int gid) {
     const int nvar = g.nvar;
     a.spikes = net->dCounters + gid;
     if (g.generated()) {
-        int st = compile_generated_head<T>(g);
+        // a network that runs in the cluster kernel never takes a stepped launch
+        int st = net->cluster.npt ? BG_OK : compile_generated_head<T>(g);
         if (st) return st;
         const bool has_tail = a.ndeliv || g.reset_kind || !g.gen_reset.empty() || g.period > 0 || a.nrec;
         const cudaKernel_t k = g.gen_kernel;
@@ -1031,35 +1066,208 @@ bool persist_direct(const HConn &c) {
            c.tgt == 0 && c.tn <= (1 << 24);
 }
 
+// The parts of that shape the persistent kernel and the cluster kernel share:
+// one group (a generated model only for the cluster kernel), its connections
+// and monitors.
+bool persist_shape(const bg_net *net) {
+    if (!net->allow_persist) return false;
+    if (net->groups.size() != 1 || !net->stdps.empty() || !net->syns.empty()) return false;
+    for (const HSpikeMon &m : net->smons)
+        if (m.gid != 0 || m.delay != 0) return false;
+    if ((int)net->stmons.size() > bg::kMaxRec) return false;
+    const HGroup &g = net->groups[0];
+    if (g.nvar < 1 || g.refr || g.period > 0 || g.emp_steps > 0 || !g.setters.empty()) return false;
+    if (g.thr_kind != BG_THR_CONST && g.thr_kind != BG_THR_VAR && g.thr_kind != BG_THR_NONE) return false;
+    if (net->conns.empty() || (int)net->conns.size() > bg::kPersistMaxPush) return false;
+    int ndirect = 0;
+    for (const HConn &c : net->conns) {
+        if (persist_direct(c)) { ++ndirect; continue; }
+        if (!c.fused_push || c.src != 0 || c.tgt != 0) return false;
+    }
+    return ndirect + (int)g.delivs.size() <= bg::kPersistMaxDeliv;
+}
+
+// Whether the network runs in the cluster kernel, and its shared memory: the
+// fewest neurons per thread (512 threads a block) for which 16 blocks hold the
+// group and everything a block keeps fits in its shared memory.  Measured
+// against the persistent kernel in bg_cluster.cuh; a forced block size of the
+// persistent kernel and the test hook of its waits mean that kernel.
+int plan_cluster(bg_net *net) {
+    bg_net::ClusterPlan best;
+    net->cluster = best;
+    if (!persist_shape(net) || net->persist_th || net->hold_block >= 0) return BG_OK;
+    const HGroup &g = net->groups[0];
+    if (!g.generated() && (!g.linear || g.nvar > 4)) return BG_OK;
+    if (g.generated() && g.nvar > bg::kMaxVars) return BG_OK;
+    const size_t ts = tsize(net);
+    int64_t tab = 0, kmax = 0;
+    int rows[2] = {3, 3};
+    for (size_t i = 0; i < net->conns.size(); ++i) {
+        HConn &c = net->conns[i];
+        if (persist_direct(c)) {
+            if (c.dir_kmax < 0) {
+                const int st = max_indegree(net, c, &c.dir_kmax);
+                if (st) return st;
+            }
+            if (c.dir_kmax >= 65535) return BG_OK;           // 16-bit counts
+            kmax += c.dir_kmax;
+            continue;
+        }
+        // a count ring, targets in 24 bits
+        if (!c.dCRing || c.tn > (1 << 24) || c.nnz <= 0) return BG_OK;
+        int dmax = 0;
+        for (uint8_t d : c.d) dmax = std::max<int>(dmax, d);
+        rows[i] = std::max(c.md, dmax + 4);
+        tab += c.tablen;
+        kmax += c.tablen - 1;
+    }
+    int dev = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return BG_OK;
+    most -= kClusterStaticSmem;
+    // one block where it holds the group, else the fewest neurons a thread
+    for (int one = 1; one >= 0; --one)
+    for (int npt : {1, 2, 4}) {
+        const int64_t bn = (int64_t)bg::kClusterThreads * npt, blocks = (g.n + bn - 1) / bn;
+        if (blocks > (one ? 1 : bg::kClusterMaxBlocks) || (blocks > 1 && bn * kmax > bg::kClusterMaxInto)) continue;
+        bg_net::ClusterPlan p;
+        p.npt = npt;
+        p.blocks = (int)blocks;
+        int64_t o = 0;
+        auto take = [&o](int64_t bytes) { const int64_t at = o; o += (bytes + 15) & ~(int64_t)15; return (int)std::min<int64_t>(at, INT32_MAX); };
+        bool direct = true;
+        int64_t syn[2] = {0, 0};
+        for (size_t c = 0; c < net->conns.size(); ++c) {
+            const HConn &q = net->conns[c];
+            const bool d = persist_direct(q);
+            direct = direct && d;
+            p.rows[c] = rows[c];
+            p.off_ring[c] = take((int64_t)rows[c] * bn * 2);
+            p.off_rows[c] = take((bn + 1) * 4);
+            // the block's synapses: at most 2^32 of them (32-bit offsets)
+            for (int64_t b = 0; b < blocks; ++b) {
+                const int64_t lo = std::min(std::max(b * bn - q.so, (int64_t)0), q.sn);
+                const int64_t hi = std::min(std::max((b + 1) * bn - q.so, (int64_t)0), q.sn);
+                syn[c] = std::max(syn[c], q.rowptr[hi] - q.rowptr[lo]);
+            }
+            if (syn[c] >= ((int64_t)1 << 32)) return BG_OK;
+        }
+        p.off_rec = take((int64_t)net->stmons.size() * (bn + 1) * 4);
+        if (o > most) continue;
+        // tables of the k-fold sums, then the synapses, where there is room
+        if (tab && o + tab * (int64_t)ts + 32 <= most)
+            for (size_t c = 0; c < net->conns.size(); ++c)
+                if (!persist_direct(net->conns[c])) p.off_tab[c] = take((int64_t)net->conns[c].tablen * ts);
+        // zero-delay networks: target indices in 16 bits (the group has at most 2^15 neurons)
+        if (direct && o + 2 * (syn[0] + syn[1]) + 32 <= most)
+            for (size_t c = 0; c < net->conns.size(); ++c) p.off_syn[c] = take(2 * syn[c]);
+        p.smem = (size_t)o;
+        net->cluster = p;
+        return BG_OK;
+    }
+    return BG_OK;
+}
+
+// The cluster kernel's launch for the planned shape, from the persistent
+// kernel's arguments.
+template <typename T>
+int build_cluster(bg_net *net, const bg::PersistArgs<T> &a, bool diag) {
+    HGroup &g = net->groups[0];
+    const bg_net::ClusterPlan &p = net->cluster;
+    bg::ClusterArgs<T> k;
+    std::memset(&k, 0, sizeof(k));
+    k.ctl = a.ctl; k.S = a.S; k.n = (int)a.n; k.npad = a.npad;
+    std::memcpy(k.A, a.A, sizeof(k.A)); std::memcpy(k.C, a.C, sizeof(k.C)); k.anz = a.anz; k.cnz = a.cnz;
+    k.linear = g.linear; k.dt = net->dt;
+    k.thr_kind = a.thr_kind; k.thr_var = a.thr_var; k.thr_var2 = a.thr_var2; k.thr_val = a.thr_val;
+    k.reset_kind = a.reset_kind; k.reset_var = a.reset_var; k.reset_var2 = a.reset_var2; k.reset_val = a.reset_val;
+    // in delivery order: the zero-delay Connections, then the DelayConnections
+    std::vector<int> order;
+    for (size_t c = 0; c < net->conns.size(); ++c)
+        if (persist_direct(net->conns[c])) order.push_back((int)c);
+    for (int c : g.delivs) order.push_back(c);
+    // onto different variables the order does not matter: ascending variables
+    if (order.size() == 2 && net->conns[order[0]].var > net->conns[order[1]].var) std::swap(order[0], order[1]);
+    k.nconn = (int)order.size();
+    // the constant form that the delivered variables, threshold and reset have
+    int pat = 0;
+    {
+        bool one = true, zero = true, up = true;
+        for (int d = 0; d < k.nconn; ++d) {
+            const int v = net->conns[order[d]].var;
+            up = up && v == d + 1; one = one && v == 1; zero = zero && v == 0;
+        }
+        pat = one ? 2 : up ? 1 : zero ? 3 : 0;
+        const bool thr = !g.gen_threshold.empty() || (a.thr_kind == BG_THR_CONST && a.thr_var == 0);
+        const bool rst = !g.gen_reset.empty() || (a.reset_kind == BG_RESET_CONST && a.reset_var == 0);
+        if (!thr || !rst) pat = 0;
+    }
+    for (int d = 0; d < k.nconn; ++d) {
+        const int c = order[d];
+        const HConn &h = net->conns[c];
+        bg::ClusterConn<T> &q = k.conn[d];
+        q.so = (int)h.so; q.sn = (int)h.sn; q.to = (int)h.to; q.tn = (int)h.tn; q.var = h.var;
+        q.direct = persist_direct(h); q.md = p.rows[c]; q.emd = h.md;
+        q.tablen = h.tablen; q.table = (const T *)h.dTable;
+        q.off_ring = p.off_ring[c]; q.off_rows = p.off_rows[c]; q.off_syn = p.off_syn[c]; q.off_tab = p.off_tab[c];
+        q.w = (T)(h.w_bits == 64 ? *(const double *)h.w.data() : (double)*(const float *)h.w.data());
+        q.rowptr = h.dRow; q.packed = a.push[c].packed; q.cring = h.dCRing; q.tnp = h.tnp;
+        q.events = a.push[c].events;
+        if (!q.packed && h.nnz > 0) return fail(BG_ESTATE, "cluster kernel: synapses not packed");
+    }
+    k.spin_limit = a.spin_limit;
+    k.split = a.lag == 2;
+    k.spikes = a.spikes;
+    k.mon_words = a.mon_words; k.mon_stride = (int)a.mon_stride;
+    k.nrec = a.nrec;
+    for (int r = 0; r < a.nrec; ++r) k.rec[r] = a.rec[r];
+    k.off_rec = p.off_rec;
+    const void *kern = nullptr;
+    if (g.generated()) {
+        const int st = compile_generated_cluster<T>(g, p.npt, p.blocks > 1, pat);
+        if (st) return st;
+        kern = (const void *)g.gen_ckernel;
+    } else {
+        kern = bg_cluster_kernel(sizeof(T) * 8, g.nvar, p.npt, diag, p.blocks > 1, pat);
+    }
+    if (!bg_cluster_fits(kern, g.gen_ckernel, p.blocks, p.smem)) {
+        if (!g.generated()) { net->cluster.npt = 0; return BG_OK; }
+        return fail(BG_ECUDA, "cluster kernel: no room for the cluster");
+    }
+    const int blocks = p.blocks;
+    const size_t smem = p.smem;
+    net->persist_used = bg::kClusterThreads;
+    net->persist = [k, kern, blocks, smem](cudaStream_t s, int nsteps) {
+        bg::ClusterArgs<T> b = k;
+        b.nsteps = nsteps;
+        return bg_cluster_launch(kern, &b, blocks, smem, s);
+    };
+    return BG_OK;
+}
+
 template <typename T>
 int build_persist(bg_net *net) {
     net->persist = nullptr;
-    if (net->groups.size() != 1 || !net->stdps.empty() || !net->syns.empty()) return BG_OK;
-    for (const HSpikeMon &m : net->smons)
-        if (m.gid != 0 || m.delay != 0) return BG_OK;
-    if ((int)net->stmons.size() > bg::kMaxRec) return BG_OK;
-
+    if (!persist_shape(net)) return BG_OK;
     const HGroup &g = net->groups[0];
-    if (!g.linear || g.nvar < 1 || g.nvar > 4 || g.refr || g.period > 0) return BG_OK;
-    if (g.generated() || g.emp_steps > 0 || !g.setters.empty()) return BG_OK;
-    if (g.thr_kind != BG_THR_CONST && g.thr_kind != BG_THR_VAR && g.thr_kind != BG_THR_NONE) return BG_OK;
-    if (net->conns.empty() || (int)net->conns.size() > bg::kPersistMaxPush) return BG_OK;
-    int min_d = 255, ndirect = 0;
+    const bool cluster = net->cluster.npt != 0;
+    if (!cluster && (!g.linear || g.nvar > 4 || g.generated())) return BG_OK;
+    int min_d = 255;
     for (const HConn &c : net->conns) {
-        if (persist_direct(c)) { ++ndirect; min_d = 0; continue; }
-        if (!c.fused_push || c.src != 0 || c.tgt != 0) return BG_OK;
+        if (persist_direct(c)) { min_d = 0; continue; }
         for (uint8_t d : c.d) min_d = std::min<int>(min_d, d);
     }
-    if (ndirect + (int)g.delivs.size() > bg::kPersistMaxDeliv) return BG_OK;
-    {
+    int th = 512;
+    if (!cluster) {
         int dev = 0, coop = 0;
         if (cudaGetDevice(&dev) != cudaSuccess) return BG_OK;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
         if (!coop) return BG_OK;
+        th = persist_threads<T>(g.n, g.nvar, net->persist_th);
+        cudaGetLastError();
+        if (!th) return BG_OK;
     }
-    const int th = persist_threads<T>(g.n, g.nvar, net->persist_th);
-    cudaGetLastError();
-    if (!th) return BG_OK;
     const int64_t bn = (int64_t)th * persist_npt(th), blocks = (g.n + bn - 1) / bn;
     net->persist_used = 0;
     // a block's synapse rows must span fewer than 2^32 entries (32-bit
@@ -1070,11 +1278,11 @@ int build_persist(bg_net *net) {
             const int64_t hi = std::min(std::max((b + 1) * bn - c.so, (int64_t)0), c.sn);
             if (c.rowptr[hi] - c.rowptr[lo] >= ((int64_t)1 << 32)) return BG_OK;
         }
-    if (net->alloc(&net->dArrived, 64) != cudaSuccess) return fail(BG_ENOMEM, "arrival counter");
+    if (!cluster && net->alloc(&net->dArrived, 64) != cudaSuccess) return fail(BG_ENOMEM, "arrival counter");
     bg::PersistArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.ctl = net->dCtl; a.S = (T *)g.dS; a.n = g.n; a.npad = g.npad; a.useC = g.useC;
-    for (int j = 0; j < g.nvar; ++j) {
+    for (int j = 0; j < g.nvar && g.linear; ++j) {
         for (int k = 0; k < g.nvar; ++k) a.A[j * g.nvar + k] = (T)g.A[j * g.nvar + k];
         a.C[j] = g.useC ? (T)g.C[j] : T(0);
     }
@@ -1086,11 +1294,10 @@ int build_persist(bg_net *net) {
     // in row t mod 3, delivered at the top of step t+1; blocks are at most
     // one step apart) and the table {0, w}
     for (HConn &c : net->conns) {
-        if (!persist_direct(c) || c.dDirRing) continue;
-        int64_t kmax = 0;
-        int st = max_indegree(net, c, &kmax);
+        if (cluster || !persist_direct(c) || c.dDirRing) continue;
+        int st = c.dir_kmax < 0 ? max_indegree(net, c, &c.dir_kmax) : BG_OK;
         if (st) return st;
-        if (kmax >= 65535) return BG_OK;                     // 16-bit counts
+        if (c.dir_kmax >= 65535) return BG_OK;               // 16-bit counts
         c.dir_md = 3;
         c.tnp = (c.tn + 1) & ~1ll;
         if (net->alloc(&c.dDirRing, (size_t)c.dir_md * c.tnp * 2) != cudaSuccess ||
@@ -1131,7 +1338,7 @@ int build_persist(bg_net *net) {
         q.cring = direct ? c.dDirRing : c.dCRing; q.tnp = c.tnp;
         // one word per synapse for the scatter: a single load (and a single
         // stream of cache lines and pages) per synapse instead of two
-        if (q.cring && c.tn <= (1 << 24) && c.nnz > 0 && c.dCols && (c.dD || direct)) {
+        if ((q.cring || (cluster && direct)) && c.tn <= (1 << 24) && c.nnz > 0 && c.dCols && (c.dD || direct)) {
             if (!c.dPacked) {
                 if (net->alloc(&c.dPacked, c.nnz * 4) != cudaSuccess) return fail(BG_ENOMEM, "packed synapses");
                 const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((c.nnz + 255) / 256, (int64_t)sm_count() * 8));
@@ -1151,7 +1358,7 @@ int build_persist(bg_net *net) {
     a.nrec = (int)net->stmons.size();
     for (int k = 0; k < a.nrec; ++k) {
         HStateMon &m = net->stmons[k];
-        if (!m.dBlkP) {
+        if (!cluster && !m.dBlkP) {
             std::vector<int32_t> lo(blocks + 1, 0);
             const int64_t w = (int64_t)m.sorted.size();
             for (int64_t b = 0, e = 0; b <= blocks; ++b) {
@@ -1184,6 +1391,12 @@ int build_persist(bg_net *net) {
     for (int j = 0; j < g.nvar; ++j)
         for (int k = 0; k < g.nvar; ++k)
             if ((((a.anz >> (j * g.nvar + k)) & 1ull) != 0) != (j == 0 || j == k)) diag = false;
+    if (cluster) {
+        const int st = build_cluster<T>(net, a, diag);
+        if (st) return st;
+        // (where the cluster does not fit the device after all: the persistent kernel)
+        return net->persist ? BG_OK : build_persist<T>(net);
+    }
     net->persist_used = th;
     net->persist = [a, blocks, nvar, arr, th, diag](cudaStream_t s, int nsteps) {
         cudaError_t e = cudaMemsetAsync(arr, 0, 64, s);
@@ -1414,8 +1627,10 @@ int bg_net_destroy(bg_net *n) {
     if (n->stream) cudaStreamSynchronize(n->stream);
     release_staging(n);
     if (n->gexec) cudaGraphExecDestroy(n->gexec);
-    for (auto &g : n->groups)
+    for (auto &g : n->groups) {
         if (g.gen_lib) cudaLibraryUnload(g.gen_lib);
+        if (g.gen_clib) cudaLibraryUnload(g.gen_clib);
+    }
     for (void *p : n->allocs) cudaFree(p);
     if (n->ev0) cudaEventDestroy(n->ev0);
     if (n->ev1) cudaEventDestroy(n->ev1);
@@ -2312,6 +2527,8 @@ static int prepare_impl(bg_net *n) {
     int st = reset_dynamic(n);
     if (st) return st;
     // ---- per-step launch list: groups, trace decay, connections slot
+    st = plan_cluster(n);
+    if (st) return st;
     for (size_t gi = 0; gi < n->groups.size(); ++gi) {
         st = n->precision == 64 ? build_group<double>(n, (int)gi) : build_group<float>(n, (int)gi);
         if (st) return st;
@@ -2882,6 +3099,8 @@ int bg_net_profile(bg_net *n, int64_t nsteps, int64_t cs0, double *ms, int64_t c
         int st0 = refresh_syn_lists(n);
         if (st0) return st0;
         *nitems = 1;
+        const long long off0 = cs0 - n->nstep;
+        BG_CUDA(cudaMemcpyAsync(&n->dCtl->clock_off, &off0, 8, cudaMemcpyHostToDevice, n->stream));
         cudaEvent_t e0, e1;
         BG_CUDA(cudaEventCreate(&e0)); BG_CUDA(cudaEventCreate(&e1));
         BG_CUDA(cudaEventRecord(e0, n->stream));
