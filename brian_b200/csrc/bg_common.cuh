@@ -96,6 +96,8 @@ struct DevCtl {
     unsigned int done;     // arrival counter of the step's last kernel
     int err;               // first error code raised on the device (0 = none)
     long long err_info;    // detail for err
+    long long mon_step;    // nstep as the step's group kernels saw it: spike monitors run beside the
+                           // step's last kernel, which advances nstep
 };
 
 #define BG_DERR_MONITOR_OVERFLOW 1

@@ -400,6 +400,7 @@ __device__ __forceinline__ void head_body(const HeadArgs<T> &a) {
     const int64_t base = (int64_t)blockIdx.x * kBlockNeurons;
     const long long nstep = a.ctl->nstep;
     const long long cs = nstep + a.ctl->clock_off;
+    if (a.update && blockIdx.x == 0 && tid == 0) a.ctl->mon_step = nstep;
     T s[kNPT][NV];
 #pragma unroll
     for (int u = 0; u < kNPT; ++u) {
@@ -1792,7 +1793,7 @@ constexpr int kMonWords = 8;
 static __global__ void __launch_bounds__(kMonThreads) k_spikemon(const MonArgs a) {
     __shared__ uint32_t sw[kMonThreads * kMonWords + kMonThreads * kMonWords / 32];   // one pad word per 32: no bank conflicts either way
     __shared__ int wcnt[kMonThreads / 32];
-    const long long nstep = a.ctl->nstep;
+    const long long nstep = a.ctl->mon_step;
     if (nstep >= a.delay && blockIdx.x == 0) {
         const long long cs = nstep + a.ctl->clock_off;
         const int32_t srel = (int32_t)(cs - *a.step_base);

@@ -20,6 +20,7 @@
 #include "bg_kernels.cuh"
 #include "bg_persist.cuh"
 #include "bg_cluster_host.h"
+#include "bg_stdplazy.cuh"
 #include "bg_synpersist.cuh"
 #include "bg_batch.cuh"
 #include "bg_rtc.h"
@@ -141,6 +142,9 @@ struct HStdp {
     // DelayConnection: trace histories of hlen steps and per-synapse lags
     bool delayed = false; int hlen = 0; std::vector<uint8_t> lag_pre, lag_post;
     double *dHpre = nullptr, *dHpost = nullptr; uint8_t *dLagPre = nullptr, *dLagPostC = nullptr;
+    // postsynaptic updates applied when a weight is needed (bg_stdplazy.cuh)
+    bool lazy = false;
+    double *dRec = nullptr; unsigned long long *dRowMask = nullptr, *dColMask = nullptr; bg::LazyCtl *dLz = nullptr;
 };
 // Synapses: incoming synapses of each target in queue order (delay
 // descending, source, synapse index), as words source | (delay+1) << 24
@@ -208,6 +212,9 @@ struct bg_net {
     std::vector<std::string> item_names;   // one per step launch
     unsigned long long *dCounters = nullptr; // [groups] spikes, then [conns] events
     std::vector<Launch> finalize_launches; // tail-only head kernels
+    // pending STDP updates: applied after every graph of steps, at the end of
+    // a run and before the masks of pending steps are full
+    std::vector<std::function<cudaError_t(cudaStream_t)>> flushes; int pending = 0;
     cudaGraphExec_t gexec = nullptr;
     // step launches [side0, side1) (the SpikeMonitors, right after the group
     // kernels) only read the spike history the group kernels wrote: in the
@@ -462,9 +469,55 @@ int sm_count() {
     return n;
 }
 
+// A dense connection with its STDP rule: one launch a step, and the flush.
+template <typename T, typename WT>
+int build_stdp_step(bg_net *net, int cid) {
+    const HConn &c = net->conns[cid];
+    const HStdp &s = net->stdps[c.stdp];
+    const HGroup &gs = net->groups[c.src], &gt = net->groups[c.tgt];
+    bg::StdpStepArgs<T> a;
+    std::memset(&a, 0, sizeof(a));
+    a.ctl = net->dCtl; a.lz = s.dLz;
+    a.hist = gs.dHist; a.depth = gs.depth; a.nwords = gs.npad / 32; a.delay = c.delay; a.so = c.so; a.sn = c.sn;
+    a.thist = gt.dHist; a.tdepth = gt.depth; a.tnwords = gt.npad / 32; a.post_delay = s.post_delay; a.to = c.to; a.tn = c.tn;
+    a.sv = (T *)gt.dS + (int64_t)c.var * gt.npad + c.to;
+    a.mod = c.mod_var >= 0 ? (const T *)gs.dS + (int64_t)c.mod_var * gs.npad + c.so : nullptr;
+    a.w = c.dW; a.A_pre = s.dApre; a.A_post = s.dApost;
+    a.a_pre = s.a_pre; a.c_pre = s.c_pre; a.a_post = s.a_post; a.c_post = s.c_post; a.Ap = s.Ap; a.Am = s.Am;
+    a.pre_set = (s.inter == BG_STDP_NEAREST || s.inter == BG_STDP_NEAREST_PRE);
+    a.post_set = (s.inter != BG_STDP_ALL);   // 'nearest_pre' writes A_post=+Am (stdp.py:500-502)
+    a.wmin = s.wmin; a.wmax = s.wmax; a.wx = s.wx; a.pre_mode = s.pre_mode; a.post_mode = s.post_mode;
+    a.rec = s.dRec; a.rowmask = s.dRowMask; a.colmask = s.dColMask;
+    a.events = net->dCounters + net->groups.size() + cid;
+    const int64_t grid = (c.tn + bg::kLazyCols - 1) / bg::kLazyCols;
+    net->item_names.push_back("stdp_step[c" + std::to_string(cid) + "]");
+    net->step_launches.push_back([a, grid](cudaStream_t st, int, int last) {
+        bg::StdpStepArgs<T> b = a; b.last = last;
+        bg::k_stdp_step<T, WT><<<(unsigned)grid, bg::kLazyThreads, 0, st>>>(b);
+        return cudaGetLastError();
+    });
+    bg::StdpFlushArgs f;
+    std::memset(&f, 0, sizeof(f));
+    f.ctl = net->dCtl; f.lz = s.dLz; f.sn = c.sn; f.tn = c.tn; f.w = c.dW;
+    f.wmin = s.wmin; f.wmax = s.wmax; f.wx = s.wx; f.mode = s.post_mode;
+    f.rec = s.dRec; f.rowmask = s.dRowMask; f.colmask = s.dColMask;
+    const int64_t bands = (c.sn + bg::kFlushRows - 1) / bg::kFlushRows;
+    const unsigned fgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(bands, (int64_t)sm_count() * 8));
+    const float flo = (float)s.wmin, fhi = (float)s.wmax;
+    const bool fast = s.post_mode == 0 && sizeof(WT) == 4 && flo >= 0.0f && flo <= fhi;
+    net->flushes.push_back([f, fgrid, fast](cudaStream_t st) {
+        if (fast) bg::k_stdp_flush<WT, true><<<fgrid, bg::kFlushThreads, 0, st>>>(f);
+        else bg::k_stdp_flush<WT, false><<<fgrid, bg::kFlushThreads, 0, st>>>(f);
+        return cudaGetLastError();
+    });
+    return BG_OK;
+}
+
 template <typename T>
 int build_conn(bg_net *net, int cid) {
     HConn &c = net->conns[cid];
+    if (c.stdp >= 0 && net->stdps[c.stdp].lazy)
+        return c.w_bits == 64 ? build_stdp_step<T, double>(net, cid) : build_stdp_step<T, float>(net, cid);
     const HGroup &gs = net->groups[c.src];
     HGroup &gt = net->groups[c.tgt];
     bg::PropArgs<T> a;
@@ -568,6 +621,7 @@ int build_stdp_pre(bg_net *net, int sid) {
 
 int build_stdp_post(bg_net *net, int sid) {
     HStdp &s = net->stdps[sid];
+    if (s.lazy) return BG_OK;
     HConn &c = net->conns[s.cid];
     const HGroup &gt = net->groups[c.tgt];
     bg::PostArgs a;
@@ -784,6 +838,7 @@ int build_spikemon(bg_net *net, int k) {
 
 int build_decay(bg_net *net, int sid) {
     HStdp &s = net->stdps[sid];
+    if (s.lazy) return BG_OK;
     const HConn &c = net->conns[s.cid];
     bg::DecayArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -856,8 +911,24 @@ int upload_state(bg_net *net, HGroup &g, int var, const double *in) {
     return BG_OK;
 }
 
+// Nothing pending: the next step is the first of a window.
+int reset_lazy(bg_net *net) {
+    net->pending = 0;
+    for (auto &s : net->stdps) {
+        if (!s.lazy) continue;
+        const HConn &c = net->conns[s.cid];
+        const bg::LazyCtl lz = {net->nstep, 0, 0};
+        BG_CUDA(cudaMemsetAsync(s.dRowMask, 0, c.sn * 16, net->stream));
+        BG_CUDA(cudaMemsetAsync(s.dColMask, 0, c.tn * 16, net->stream));
+        BG_CUDA(cudaMemcpyAsync(s.dLz, &lz, sizeof(lz), cudaMemcpyHostToDevice, net->stream));
+    }
+    return BG_OK;
+}
+
 int reset_dynamic(bg_net *net) {
     net->syn_lists_stale = true;
+    int lst = reset_lazy(net);
+    if (lst) return lst;
     for (auto &g : net->groups) {
         BG_CUDA(cudaMemsetAsync(g.dHist, 0, (size_t)g.depth * (g.npad / 32) * 4, net->stream));
         if (g.dNext) {
@@ -2416,6 +2487,15 @@ static int prepare_impl(bg_net *n) {
                     break;
                 }
         }
+        // on a dense connection the rule's kernels share one launch and the
+        // postsynaptic updates wait (the trace records of 64 steps: 512 bytes a source)
+        s.lazy = s.fused && c.dense && c.sn > 0 && c.tn > 0 && c.sn * bg::kLazySteps * 8 <= ((int64_t)1 << 30);
+        if (s.lazy) {
+            if (n->alloc(&s.dRec, (size_t)c.sn * bg::kLazySteps * 8) != cudaSuccess ||
+                n->alloc(&s.dRowMask, (size_t)c.sn * 16) != cudaSuccess || n->alloc(&s.dColMask, (size_t)c.tn * 16) != cudaSuccess ||
+                n->alloc(&s.dLz, sizeof(bg::LazyCtl)) != cudaSuccess)
+                return fail(BG_ENOMEM, "STDP pending updates");
+        }
     }
     for (auto &m : n->smons) {
         m.cap = std::max<int64_t>(1024, m.n * (n->chunk_steps + 1));
@@ -2610,20 +2690,35 @@ static int refresh_syn_lists(bg_net *n) {
     return BG_OK;
 }
 
+// the pending STDP updates of the steps so far, on the network's stream
+static int launch_flushes(bg_net *n) {
+    for (auto &f : n->flushes) {
+        cudaError_t e = f(n->stream);
+        if (e != cudaSuccess) return fail(BG_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
+        n->launches++;
+    }
+    n->pending = 0;
+    return BG_OK;
+}
+
 static int launch_step(bg_net *n, int tail) {
+    if (!n->flushes.empty() && n->pending >= bg::kLazySteps) { int st = launch_flushes(n); if (st) return st; }
     const size_t k = n->step_launches.size();
     for (size_t i = 0; i < k; ++i) {
         cudaError_t e = n->step_launches[i](n->stream, tail, i + 1 == k);
         if (e != cudaSuccess) return fail(BG_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     }
     n->launches += (int64_t)k;
+    n->pending++;
     return BG_OK;
 }
 
 // one step into the graph being captured, the side launches on the side
-// stream (forked after the group kernels, joined before the last launch)
-static int capture_step_forked(bg_net *n) {
+// stream (forked after the group kernels; joined before the next step's first
+// launch, whose group kernels overwrite what they read)
+static int capture_step_forked(bg_net *n, bool first) {
     const size_t k = n->step_launches.size();
+    if (!first) BG_CUDA(cudaStreamWaitEvent(n->stream, n->ev_join, 0));
     for (size_t i = 0; i < k; ++i) {
         cudaStream_t st = n->stream;
         if (i == n->side0) {
@@ -2632,7 +2727,6 @@ static int capture_step_forked(bg_net *n) {
         }
         if (i >= n->side0 && i < n->side1) st = n->side;
         if (i == n->side1) BG_CUDA(cudaEventRecord(n->ev_join, n->side));
-        if (i + 1 == k) BG_CUDA(cudaStreamWaitEvent(n->stream, n->ev_join, 0));
         cudaError_t e = n->step_launches[i](st, 1, i + 1 == k);
         if (e != cudaSuccess) return fail(BG_ECUDA, std::string("kernel launch: ") + cudaGetErrorString(e));
     }
@@ -2650,11 +2744,16 @@ static int ensure_graph(bg_net *n) {
         BG_CUDA(cudaEventCreateWithFlags(&n->ev_join, cudaEventDisableTiming));
     }
     cudaGraph_t graph;
+    const int64_t launches0 = n->launches;
+    n->pending = 0;
     BG_CUDA(cudaStreamBeginCapture(n->stream, cudaStreamCaptureModeThreadLocal));
     int st = BG_OK;
-    for (int s = 0; s < kGraphSteps && st == BG_OK; ++s) st = fork ? capture_step_forked(n) : launch_step(n, 1);
+    for (int s = 0; s < kGraphSteps && st == BG_OK; ++s) st = fork ? capture_step_forked(n, s == 0) : launch_step(n, 1);
+    if (st == BG_OK && fork && cudaStreamWaitEvent(n->stream, n->ev_join, 0) != cudaSuccess)
+        st = fail(BG_ECUDA, "graph capture: join");
+    if (st == BG_OK) st = launch_flushes(n);
     cudaError_t e = cudaStreamEndCapture(n->stream, &graph);
-    n->launches -= (int64_t)kGraphSteps * (int64_t)n->step_launches.size();
+    n->launches = launches0;
     if (st) return st;
     if (e != cudaSuccess) return fail(BG_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(&n->gexec, graph, 0);
@@ -2754,8 +2853,11 @@ static int net_run_steps(bg_net *n, int64_t nsteps, int64_t cs0) {
         int64_t k = 0;
         if (done == 0) { st = launch_step(n, 0); if (st) return st; k = 1; }
         while (c - k >= kGraphSteps) {
+            // the graph's own steps and those before it fit the masks of pending steps
+            if (!n->flushes.empty() && n->pending + kGraphSteps > bg::kLazySteps && (st = launch_flushes(n))) return st;
             BG_CUDA(cudaGraphLaunch(n->gexec, n->stream));
-            n->launches += (int64_t)kGraphSteps * (int64_t)n->step_launches.size();
+            n->launches += (int64_t)kGraphSteps * (int64_t)n->step_launches.size() + (int64_t)n->flushes.size();
+            n->pending = 0;
             k += kGraphSteps;
         }
         for (; k < c; ++k) { st = launch_step(n, 1); if (st) return st; }
@@ -2768,6 +2870,7 @@ static int net_run_steps(bg_net *n, int64_t nsteps, int64_t cs0) {
                 if (e != cudaSuccess) return fail(BG_ECUDA, cudaGetErrorString(e));
                 n->launches++;
             }
+            if (n->pending && (st = launch_flushes(n))) return st;
         }
         BG_CUDA(cudaEventRecord(n->ev1, n->stream));
         BG_CUDA(cudaEventSynchronize(n->ev1));
@@ -2971,6 +3074,7 @@ int bg_net_load_state(bg_net *n, const void *buf, int64_t bytes) {
     if (r.left) { n->failed = true; return fail(BG_EINVAL, "state has trailing bytes; the network must be rebuilt"); }
     n->nstep = nstep;
     n->syn_lists_stale = true;
+    { int lst = reset_lazy(n); if (lst) return lst; }
     long long ns = nstep;
     BG_CUDA(cudaMemcpy(&n->dCtl->nstep, &ns, 8, cudaMemcpyHostToDevice));
     for (auto &m : n->stmons) BG_CUDA(cudaMemcpy(m.dRowBase, &m.rows_done, 8, cudaMemcpyHostToDevice));
@@ -3134,6 +3238,7 @@ int bg_net_profile(bg_net *n, int64_t nsteps, int64_t cs0, double *ms, int64_t c
         BG_CUDA(cudaEventSynchronize(ev[k]));
         for (size_t i = 0; i < k; ++i) { float t = 0; cudaEventElapsedTime(&t, ev[i], ev[i + 1]); acc[i] += t; }
         n->launches += (int64_t)k;
+        if (!n->flushes.empty() && (++n->pending == kGraphSteps || s + 1 == nsteps) && st == BG_OK) st = launch_flushes(n);
     }
     n->nstep += nsteps;
     for (auto &f : n->finalize_launches) { cudaError_t e = f(n->stream, 1, 0); if (e != cudaSuccess && st == BG_OK) st = fail(BG_ECUDA, cudaGetErrorString(e)); }
