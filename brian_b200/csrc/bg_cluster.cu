@@ -1,4 +1,9 @@
 // bg_cluster.cu -- launch of the cluster kernel (bg_cluster.cuh).
+#include <map>
+#include <mutex>
+#include <set>
+#include <utility>
+
 #include "bg_cluster_host.h"
 
 namespace {
@@ -33,14 +38,33 @@ bool bg_cluster_fits(const void *kernel, cudaKernel_t generated, int blocks, siz
         return generated ? cudaKernelSetAttributeForDevice(generated, at, v, dev) : cudaFuncSetAttribute(kernel, at, v);
     };
     // the limits belong to the kernel, not to this network: the largest there
-    // is, so that no other network's call lowers them
-    cudaLaunchAttribute at[1];
-    cudaLaunchConfig_t c = config(at, blocks, smem, nullptr);
-    const bool ok = set(cudaFuncAttributeMaxDynamicSharedMemorySize, most - kClusterStaticSmem) == cudaSuccess &&
-                    set(cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&n, generated ? (const void *)generated : kernel, &c) == cudaSuccess && n >= 1;
-    cudaGetLastError();
-    return ok;
+    // is, so that no other network's call lowers them.  Built-in kernels are
+    // set once; whether the device places a cluster of that many blocks with
+    // that much shared memory is asked once per size (the query takes
+    // milliseconds, and clusters of up to 8 blocks are always placed).
+    static std::mutex mutex;
+    static std::set<std::pair<int, const void *>> ready;
+    static std::map<std::pair<int, int>, bool> placed;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (generated || !ready.count({dev, kernel})) {
+        if (set(cudaFuncAttributeMaxDynamicSharedMemorySize, most - kClusterStaticSmem) != cudaSuccess ||
+            set(cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (!generated) ready.insert({dev, kernel});
+    }
+    if ((int64_t)smem > most - kClusterStaticSmem) return false;
+    if (blocks <= 8) return true;
+    auto it = placed.find({dev, blocks});
+    if (it == placed.end()) {
+        cudaLaunchAttribute at[1];
+        cudaLaunchConfig_t c = config(at, blocks, (size_t)(most - kClusterStaticSmem), nullptr);
+        const bool ok = cudaOccupancyMaxActiveClusters(&n, generated ? (const void *)generated : kernel, &c) == cudaSuccess && n >= 1;
+        cudaGetLastError();
+        it = placed.emplace(std::make_pair(dev, blocks), ok).first;
+    }
+    return it->second;
 }
 
 cudaError_t bg_cluster_launch(const void *kernel, const void *args, int blocks, size_t smem, cudaStream_t s) {
