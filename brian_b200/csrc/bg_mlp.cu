@@ -3,20 +3,22 @@
 // over the fitted parameters (5 means, 5 log standard deviations), trained by
 // Gaussian negative log-likelihood with Adam.
 //
-// Every matrix product, forward and backward, runs in one hand-written
-// tcgen05 kernel (bg_umma.cuh) with BF16 operands and FP32 accumulation:
+// Every matrix product runs on the tensor cores (tcgen05) with BF16 operands
+// and FP32 accumulation, in three launches (bg_mlpchain.cuh):
 //
-//   forward   H_l = relu(H_{l-1} W_l^T + b_l)          A = H_{l-1}, B = W_l
-//   backward  G_l = (G_{l+1} W_{l+1}) * [H_l > 0]       A = G_{l+1}, B = W_{l+1}^T
-//             dW_l = G_l^T H_{l-1}                      A = G_l^T,  B = H_{l-1}^T
+//   forward   H_l = relu(H_{l-1} W_l^T + b_l)     128 batch rows through all layers
+//   backward  G_l = (G_{l+1} W_{l+1}) * [H_l > 0]  likewise
+//   weights   dW_l = G_l^T H_{l-1}                 all four, with the bias sums
 //
-// so each layer keeps its activations and gradients in both layouts (the
-// epilogues write the transposed copy), and the weights exist as FP32
-// master copies plus BF16 copies in both layouts, refreshed by the Adam
-// kernel.  The output layer is padded from 10 to 64 rows (zero rows, zero
-// gradients) so every K is a multiple of 64.  Weight gradients split the
-// batch reduction over grid.z and are summed in a fixed order by the Adam
-// kernel (deterministic).
+// The chains write each activation and gradient once, row-major; the weight
+// gradients read them as MN-major operands, so there are no transposed copies
+// of them.  The weights exist as FP32 master copies plus BF16 copies in both
+// layouts, written by the Adam kernel.  The output layer is padded from 10 to
+// 64 rows (zero rows, zero gradients) so every K is a multiple of 64.  Weight
+// gradients split the batch reduction eight ways and the slices are summed in
+// a fixed order by the Adam kernel (deterministic).  A training step is six
+// launches: gather, forward, loss, backward, weight gradients, Adam (16384
+// rows: 351 -> 173 us a step with one product per launch before).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cub/device/device_radix_sort.cuh>
@@ -30,7 +32,7 @@
 #include <vector>
 
 #include "bg_common.cuh"
-#include "bg_umma.cuh"
+#include "bg_mlpchain.cuh"
 #include "../../include/brian_b200.h"
 
 namespace {
@@ -46,70 +48,89 @@ int fail(int code, const std::string &m) { return bg_internal_fail(code, m.c_str
 
 constexpr int kIn = 64, kHid = 512, kOutPad = 64, kNLayer = 4;
 constexpr int kSplits = 8;
-// Output tile width of the network's GEMMs: 64 columns keeps 256 CTAs in
-// flight per 4096-row product (two or three per SM), so one CTA's load
-// latency overlaps another's tensor-core work.
-constexpr int kNT = 64;
 
 typedef __nv_bfloat16 bf16;
 
 // ------------------------------------------------------------------ kernels
-// Batch rows idx[0..B) of the normalised training set -> X (bf16), X^T, Y.
-__global__ void k_gather(const float *Xall, const float *Yall, const int64_t *idx, int B, int ydim, bf16 *X, bf16 *XT,
-                         float *Y) {
-    const int b = blockIdx.x;
-    const int64_t r = idx[b];
-    for (int j = threadIdx.x; j < kIn; j += blockDim.x) {
-        const bf16 v = __float2bfloat16_rn(Xall[r * kIn + j]);
-        X[(int64_t)b * kIn + j] = v;
-        XT[(int64_t)j * B + b] = v;
-    }
-    for (int j = threadIdx.x; j < ydim; j += blockDim.x) Y[(int64_t)b * ydim + j] = Yall[r * ydim + j];
+// Batch rows of the normalised training set -> X (bf16), Y.  Row b of the batch
+// is row order[base + b], base = B * batch_index (a device counter, so the
+// gather can sit in a captured graph; null: 0).  Eight threads a row, 32 rows a
+// block: each thread two 16-byte loads and one 16-byte store, where one block a
+// row was bound by the launch of its blocks (16384 rows: 12.5 -> 5.8 us).
+__global__ void __launch_bounds__(256) k_gather(const float *Xall, const float *Yall, const int64_t *order,
+                                                const int64_t *batch_index, int B, int ydim, bf16 *X, float *Y) {
+    umma::pdl_launch_dependents();
+    umma::pdl_wait();
+    const int b = blockIdx.x * 32 + (threadIdx.x >> 3), j = (threadIdx.x & 7) * 8;
+    if (b >= B) return;
+    const int64_t r = order[(batch_index ? *batch_index * B : 0) + b];
+    const float4 lo = *reinterpret_cast<const float4 *>(Xall + r * kIn + j);
+    const float4 hi = *reinterpret_cast<const float4 *>(Xall + r * kIn + j + 4);
+    __nv_bfloat162 h[4] = {__floats2bfloat162_rn(lo.x, lo.y), __floats2bfloat162_rn(lo.z, lo.w),
+                           __floats2bfloat162_rn(hi.x, hi.y), __floats2bfloat162_rn(hi.z, hi.w)};
+    *reinterpret_cast<uint4 *>(X + (int64_t)b * kIn + j) = *reinterpret_cast<const uint4 *>(h);
+    for (int q = threadIdx.x & 7; q < ydim; q += 8) Y[(int64_t)b * ydim + q] = Yall[r * ydim + q];
 }
 
 // Gaussian NLL per sample, mean over the batch:
 //   sum_d 0.5 ((y_d - mu_d) e^{-s_d})^2 + s_d,  s = clamp(log sigma, -7, 7)
-// gradients (already divided by B) into dOUT (bf16, both layouts; the
-// padded columns stay zero from allocation) and per-block column sums of the
+// gradients (already divided by B) into dOUT (bf16; the padded columns stay
+// zero from allocation) and per-block column sums of the
 // bf16 gradients into colsum[blockIdx.x][64] (the output bias gradient).
-__global__ void __launch_bounds__(256) k_nll(const float *OUT, const float *Y, int B, int ydim, bf16 *dO, bf16 *dOT,
+__global__ void __launch_bounds__(256) k_nll(const float *OUT, const float *Y, int B, int ydim, bf16 *dO,
                                              float *colsum, float *loss_sum) {
     umma::pdl_launch_dependents();
     umma::pdl_wait();
     constexpr int kMaxY = kOutPad / 2;
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ float red[8][kOutPad];
     __shared__ float lred[8];
     float l = 0.f;
-    float gcol[kOutPad];
+    const float inv_b = 1.0f / (float)B;
+    // (chunks of kYc outputs, so that their loads and the shuffles of their sums
+    // overlap; every index below is a constant of the unrolled code)
+    constexpr int kYc = 5;
+    for (int j0 = 0; j0 < ydim; j0 += kYc) {
+        float mu[kYc], sr[kYc], y[kYc], gm[kYc], gs[kYc];
 #pragma unroll
-    for (int j = 0; j < kOutPad; ++j) gcol[j] = 0.f;
-    if (b < B) {
-        const float inv_b = 1.0f / (float)B;
-        for (int j = 0; j < ydim && j < kMaxY; ++j) {
-            const float mu = OUT[(int64_t)b * kOutPad + j];
-            const float sr = OUT[(int64_t)b * kOutPad + ydim + j];
-            const float s = fminf(fmaxf(sr, -7.f), 7.f);
-            const float r = (Y[(int64_t)b * ydim + j] - mu) * expf(-s);
-            l += 0.5f * r * r + s;
-            const bf16 g = __float2bfloat16_rn(-r * expf(-s) * inv_b);                                  // d/d mu
-            const bf16 gs = __float2bfloat16_rn((sr > -7.f && sr < 7.f) ? (1.f - r * r) * inv_b : 0.f);  // d/d log sigma
-            dO[(int64_t)b * kOutPad + j] = g;
-            dO[(int64_t)b * kOutPad + ydim + j] = gs;
-            dOT[(int64_t)j * B + b] = g;
-            dOT[(int64_t)(ydim + j) * B + b] = gs;
-            gcol[j] = __bfloat162float(g);
-            gcol[ydim + j] = __bfloat162float(gs);
+        for (int q = 0; q < kYc; ++q) {
+            const int j = j0 + q;
+            const bool on = b < B && j < ydim && j < kMaxY;
+            mu[q] = on ? OUT[(int64_t)b * kOutPad + j] : 0.f;
+            sr[q] = on ? OUT[(int64_t)b * kOutPad + ydim + j] : 0.f;
+            y[q] = on ? Y[(int64_t)b * ydim + j] : 0.f;
         }
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-    for (int j = 0; j < kOutPad; ++j) {
-        if (j >= 2 * ydim) break;
-        float v = gcol[j];
+        for (int q = 0; q < kYc; ++q) {
+            const int j = j0 + q;
+            gm[q] = gs[q] = 0.f;
+            if (b < B && j < ydim && j < kMaxY) {
+                const float s = fminf(fmaxf(sr[q], -7.f), 7.f);
+                const float r = (y[q] - mu[q]) * expf(-s);
+                l += 0.5f * r * r + s;
+                const bf16 g = __float2bfloat16_rn(-r * expf(-s) * inv_b);                                        // d/d mu
+                const bf16 gg = __float2bfloat16_rn((sr[q] > -7.f && sr[q] < 7.f) ? (1.f - r * r) * inv_b : 0.f);  // d/d log sigma
+                dO[(int64_t)b * kOutPad + j] = g;
+                dO[(int64_t)b * kOutPad + ydim + j] = gg;
+                gm[q] = __bfloat162float(g);
+                gs[q] = __bfloat162float(gg);
+            }
+        }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-        if (lane == 0) red[warp][j] = v;
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (int q = 0; q < kYc; ++q) {
+                gm[q] += __shfl_xor_sync(0xffffffffu, gm[q], off);
+                gs[q] += __shfl_xor_sync(0xffffffffu, gs[q], off);
+            }
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < kYc; ++q)
+                if (j0 + q < ydim) {
+                    red[warp][j0 + q] = gm[q];
+                    red[warp][ydim + j0 + q] = gs[q];
+                }
     }
     float lv = l;
 #pragma unroll
@@ -148,100 +169,69 @@ struct AdamSeg {
 struct AdamAll {
     AdamSeg seg[2 * kNLayer];
     int64_t off[2 * kNLayer + 1];
+    int blk0[2 * kNLayer + 1];     // first block of each segment: 32 x 32 tiles of a weight, 256 entries of a bias
     const int64_t *step;
     float lr, b1, b2, eps;
     float scale;                   // gradient multiplier (1: exact; 1/ranks after a summing all-reduce)
 };
-__global__ void k_adam_all(const __grid_constant__ AdamAll a) {
+// The sum of entry i's partial slices, in slice order.
+__device__ __forceinline__ float sum_slices(const AdamSeg &sg, int64_t i) {
+    float g = 0.f;
+    if (sg.splits == kSplits) {
+#pragma unroll
+        for (int s = 0; s < kSplits; ++s) g += sg.grad[s * sg.split_stride + i];
+    } else {
+        for (int s = 0; s < sg.splits; ++s) g += sg.grad[s * sg.split_stride + i];
+    }
+    return g;
+}
+__device__ __forceinline__ float adam_entry(const AdamAll &a, const AdamSeg &sg, int64_t i, float c1, float c2) {
+    const float g = sum_slices(sg, i) * a.scale;
+    const float mi = a.b1 * sg.m[i] + (1.f - a.b1) * g;
+    const float vi = a.b2 * sg.v[i] + (1.f - a.b2) * g * g;
+    sg.m[i] = mi;
+    sg.v[i] = vi;
+    const float p = sg.P[i] - a.lr * (mi / c1) / (sqrtf(vi / c2) + a.eps);
+    sg.P[i] = p;
+    return p;
+}
+// Bound by the 28 bytes an entry moves plus 4 per partial slice.  A block updates a
+// 32 x 32 tile of one weight, so that its bf16 copy and (through shared memory) the
+// transposed one are written in whole rows by the same launch: 13.6 us and 5.7 us
+// of a second one before, 13.2 us now.
+__global__ void __launch_bounds__(256) k_adam_all(const __grid_constant__ AdamAll a) {
     umma::pdl_launch_dependents();
     umma::pdl_wait();
-    const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i0 >= a.off[2 * kNLayer]) return;
+    __shared__ float corr[2];
+    __shared__ bf16 tile[32][33];
+    if (threadIdx.x < 2) corr[threadIdx.x] = 1.f - powf(threadIdx.x ? a.b2 : a.b1, (float)*a.step);
+    __syncthreads();
     int k = 0;
 #pragma unroll
-    for (int q = 1; q < 2 * kNLayer; ++q) k += i0 >= a.off[q] ? 1 : 0;
+    for (int q = 1; q < 2 * kNLayer; ++q) k += (int)blockIdx.x >= a.blk0[q] ? 1 : 0;
     const AdamSeg &sg = a.seg[k];
-    const int64_t i = i0 - a.off[k];
-    const int r = (int)(i / sg.cols);
-    if (r < sg.rows_train) {
-        const float t = (float)*a.step;
-        const float c1 = 1.f - powf(a.b1, t), c2 = 1.f - powf(a.b2, t);
-        float g = 0.f;
-        for (int s = 0; s < sg.splits; ++s) g += sg.grad[s * sg.split_stride + i];
-        g *= a.scale;
-        const float mi = a.b1 * sg.m[i] + (1.f - a.b1) * g;
-        const float vi = a.b2 * sg.v[i] + (1.f - a.b2) * g * g;
-        sg.m[i] = mi;
-        sg.v[i] = vi;
-        sg.P[i] -= a.lr * (mi / c1) / (sqrtf(vi / c2) + a.eps);
+    const int blk = (int)blockIdx.x - a.blk0[k];
+    const float c1 = corr[0], c2 = corr[1];
+    if (!sg.Pb) {
+        const int i = blk * 256 + (int)threadIdx.x;
+        if (i < sg.rows_train) adam_entry(a, sg, i, c1, c2);
+        return;
     }
-    if (sg.Pb) sg.Pb[i] = __float2bfloat16_rn(sg.P[i]);   // the transposed copy: k_transpose_all
-}
-
-// The transposed bf16 copies of the updated weights (PbT[c][r] = Pb[r][c]),
-// 32 x 32 tiles through shared memory so that both the reads and the writes
-// are coalesced; block b is a tile of the first segments with a PbT.
-__global__ void __launch_bounds__(256) k_transpose_all(const __grid_constant__ AdamAll a) {
-    umma::pdl_launch_dependents();
-    umma::pdl_wait();
-    __shared__ bf16 tile[32][33];
-    int b = blockIdx.x, k = 0;
-    for (; k < 2 * kNLayer; ++k) {
-        const AdamSeg &sg = a.seg[k];
-        if (!sg.PbT) continue;
-        const int nt = ((sg.rows + 31) / 32) * ((sg.cols + 31) / 32);
-        if (b < nt) break;
-        b -= nt;
-    }
-    if (k == 2 * kNLayer) return;
-    const AdamSeg &sg = a.seg[k];
-    const int tcols = (sg.cols + 31) / 32;
-    const int r0 = (b / tcols) * 32, c0 = (b % tcols) * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;
+    const int tcols = sg.cols / 32, r0 = (blk / tcols) * 32, c0 = (blk % tcols) * 32;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
     for (int j = 0; j < 32; j += 8) {
-        const int r = r0 + ty + j, c = c0 + tx;
-        if (r < sg.rows && c < sg.cols) tile[ty + j][tx] = sg.Pb[(int64_t)r * sg.cols + c];
+        const int r = r0 + ty + j;
+        const int64_t i = (int64_t)r * sg.cols + c0 + tx;
+        const bf16 p = __float2bfloat16_rn(r < sg.rows_train ? adam_entry(a, sg, i, c1, c2) : sg.P[i]);
+        sg.Pb[i] = p;
+        tile[ty + j][tx] = p;
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-        const int c = c0 + ty + j, r = r0 + tx;
-        if (r < sg.rows && c < sg.cols) sg.PbT[(int64_t)c * sg.rows + r] = tile[tx][ty + j];
-    }
+    for (int j = 0; j < 32; j += 8) sg.PbT[(int64_t)(c0 + ty + j) * sg.rows + r0 + tx] = tile[tx][ty + j];
 }
-
-// The bias gradients, each the sum of its layer's column-sum partials (one
-// per 32 or 256 batch rows), in one fixed order: block b sums 32 columns of
-// one layer, warp w the partials w, w + 8, ... of them (coalesced rows), and
-// warp 0 adds the eight warp sums in warp order.
-struct BiasRed {
-    const float *p[kNLayer]; int nblk[kNLayer], ld[kNLayer], rows[kNLayer];
-    int blk0[kNLayer + 1];          // first block of each layer
-    float *out;                     // [kNLayer][kHid]
-};
-__global__ void __launch_bounds__(256) k_bias_reduce(const __grid_constant__ BiasRed r) {
-    umma::pdl_launch_dependents();
-    umma::pdl_wait();
-    __shared__ float red[8][32];
-    int l = 0;
-    while (l + 1 < kNLayer && (int)blockIdx.x >= r.blk0[l + 1]) ++l;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i = ((int)blockIdx.x - r.blk0[l]) * 32 + lane;
-    float g = 0.f;
-    if (i < r.rows[l]) {
-#pragma unroll 8
-        for (int s = warp; s < r.nblk[l]; s += 8) g += r.p[l][(int64_t)s * r.ld[l] + i];
-    }
-    red[warp][lane] = g;
-    __syncthreads();
-    if (warp == 0 && i < r.rows[l]) {
-        float t = red[0][lane];
-#pragma unroll
-        for (int w = 1; w < 8; ++w) t += red[w][lane];
-        r.out[l * kHid + i] = t;
-    }
-}
+static_assert(kIn % 32 == 0 && kHid % 32 == 0 && kOutPad % 32 == 0, "Adam's tiles are whole");
 
 // The gradient of every tensor as one flat vector in the optimiser's segment
 // order (W0, b0, W1, b1, ...): each entry the sum of its partial slices in
@@ -255,13 +245,12 @@ __global__ void k_grad_flat(const __grid_constant__ AdamAll a, float *flat) {
     for (int q = 1; q < 2 * kNLayer; ++q) k += i0 >= a.off[q] ? 1 : 0;
     const AdamSeg &sg = a.seg[k];
     const int64_t i = i0 - a.off[k];
-    float g = 0.f;
-    for (int s = 0; s < sg.splits; ++s) g += sg.grad[s * sg.split_stride + i];
-    flat[i0] = g;
+    flat[i0] = sum_slices(sg, i);
 }
 
-// One training step's bookkeeping: the batch index within the epoch and the
-// optimiser step, advanced after the step's kernels.
+// The bookkeeping of a step whose gradients come from outside: the batch index
+// within the epoch and the optimiser step (a training step's own are advanced by
+// the weight-gradient kernel).
 __global__ void k_step_advance(int64_t *batch_index, int64_t *opt_step) {
     umma::pdl_launch_dependents();
     umma::pdl_wait();
@@ -277,20 +266,6 @@ __global__ void k_perm_keys(uint64_t seed, int64_t epoch, int64_t n, unsigned lo
         keys[i] = ((unsigned long long)c[0] << 32) | c[1];
         vals[i] = i;
     }
-}
-
-// Batch rows idx[base .. base+B) with base = B * batch_index (a device
-// counter, so the gather can sit in a captured graph).
-__global__ void k_gather_at(const float *Xall, const float *Yall, const int64_t *perm, const int64_t *batch_index,
-                            int B, int ydim, bf16 *X, bf16 *XT, float *Y) {
-    const int b = blockIdx.x;
-    const int64_t r = perm[*batch_index * B + b];
-    for (int j = threadIdx.x; j < kIn; j += blockDim.x) {
-        const bf16 v = __float2bfloat16_rn(Xall[r * kIn + j]);
-        X[(int64_t)b * kIn + j] = v;
-        XT[(int64_t)j * B + b] = v;
-    }
-    for (int j = threadIdx.x; j < ydim; j += blockDim.x) Y[(int64_t)b * ydim + j] = Yall[r * ydim + j];
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no
@@ -329,17 +304,17 @@ bool tile_map(CUtensorMap *m, const bf16 *base, int rows, int cols, int ld, int 
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NT, int EPI, bool TMA>
+template <int NT, bool TMA>
 int launch_gemm_as(const umma::GemmArgs &g, int splits, cudaStream_t st, const CUtensorMap &ta,
                    const CUtensorMap &tb) {
     static bool attr_set = false;
     constexpr size_t smem = umma::smem_bytes<NT>();
     if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_gemm<NT, EPI, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MCK(cudaFuncSetAttribute(umma::k_gemm<NT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
     dim3 grid((unsigned)((g.M + umma::kM - 1) / umma::kM), (unsigned)((g.N + NT - 1) / NT), (unsigned)splits);
-    umma::k_gemm<NT, EPI, TMA><<<grid, umma::kThreads, smem, st>>>(g, ta, tb);
+    umma::k_gemm<NT, TMA><<<grid, umma::kThreads, smem, st>>>(g, ta, tb);
     MCK(cudaGetLastError());
     return BG_OK;
 }
@@ -370,19 +345,19 @@ int sm_count_mlp() {
 }
 
 // The persistent warp-specialised kernel over all tiles of the product.
-template <int NT, int EPI>
+template <int NT>
 int launch_gemm_persistent(const umma::GemmArgs &g, int splits, cudaStream_t st, const CUtensorMap &ta,
                            const CUtensorMap &tb) {
     static bool attr_set = false;
     constexpr size_t smem = umma::psmem_bytes<NT>();
     if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_gemm_p<NT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        MCK(cudaFuncSetAttribute(umma::k_gemm_p<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr_set = true;
     }
     const int tiles_m = (g.M + umma::kM - 1) / umma::kM, tiles_n = (g.N + NT - 1) / NT;
     const int ntiles = tiles_m * tiles_n * splits;
     const int grid = std::max(1, std::min(ntiles, sm_count_mlp()));
-    MCK(launch_pdl(umma::k_gemm_p<NT, EPI>, dim3(grid), dim3(umma::kPThreads), smem, st, g, ta, tb, tiles_m, tiles_n,
+    MCK(launch_pdl(umma::k_gemm_p<NT>, dim3(grid), dim3(umma::kPThreads), smem, st, g, ta, tb, tiles_m, tiles_n,
                    splits));
     return BG_OK;
 }
@@ -390,17 +365,42 @@ int launch_gemm_persistent(const umma::GemmArgs &g, int splits, cudaStream_t st,
 // TMA-fed persistent kernel when both operands allow a tensor map (16-byte
 // aligned rows, K a multiple of 8) and every split has K-chunks, else the
 // one-tile-per-CTA kernel with cp.async stages.
-template <int NT, int EPI>
+template <int NT>
 int launch_gemm(const umma::GemmArgs &g, int splits, cudaStream_t st) {
     CUtensorMap ta, tb;
     memset(&ta, 0, sizeof ta);
     memset(&tb, 0, sizeof tb);
     if (g.k_per_split >= umma::kKc && g.k_per_split % umma::kKc == 0 && (long long)g.k_per_split * splits == g.K &&
         tile_map(&ta, g.A, g.M, g.K, g.lda, umma::kM, true) && tile_map(&tb, g.B, g.N, g.K, g.ldb, NT, true))
-        return launch_gemm_persistent<NT, EPI>(g, splits, st, ta, tb);
+        return launch_gemm_persistent<NT>(g, splits, st, ta, tb);
     memset(&ta, 0, sizeof ta);
     memset(&tb, 0, sizeof tb);
-    return launch_gemm_as<NT, EPI, false>(g, splits, st, ta, tb);
+    return launch_gemm_as<NT, false>(g, splits, st, ta, tb);
+}
+
+template <bool BWD>
+int launch_chain(const umma::ChainArgs &g, const umma::ChainMaps &m, cudaStream_t st) {
+    static bool attr_set = false;
+    constexpr size_t smem = umma::chain_smem_bytes();
+    if (!attr_set) {
+        MCK(cudaFuncSetAttribute(umma::k_mlp_chain<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set = true;
+    }
+    const int grid = std::max(1, std::min(g.rows / umma::kM, sm_count_mlp()));
+    MCK(launch_pdl(umma::k_mlp_chain<BWD>, dim3(grid), dim3(umma::kPThreads), smem, st, g, m));
+    return BG_OK;
+}
+
+int launch_weight_gradients(const umma::DwArgs &g, const umma::DwMaps &m, cudaStream_t st) {
+    static bool attr_set = false;
+    constexpr size_t smem = sizeof(umma::DwSmem);
+    if (!attr_set) {
+        MCK(cudaFuncSetAttribute(umma::k_weight_gradients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        attr_set = true;
+    }
+    const int grid = std::max(1, std::min(g.units, sm_count_mlp()));
+    MCK(launch_pdl(umma::k_weight_gradients, dim3(grid), dim3(umma::kPThreads), smem, st, g, m));
+    return BG_OK;
 }
 
 umma::GemmArgs gemm_args(const bf16 *A, int lda, const bf16 *B, int ldb, int M, int N, int K, int *err) {
@@ -414,7 +414,6 @@ umma::GemmArgs gemm_args(const bf16 *A, int lda, const bf16 *B, int ldb, int M, 
     g.lda = lda;
     g.ldb = ldb;
     g.k_per_split = K;
-    g.n_valid = N;
     g.err = err;
     return g;
 }
@@ -459,10 +458,17 @@ struct bg_mlp {
     float *cs[kNLayer] = {};              // bias-gradient partials per layer [row blocks][512]
     float *gbias = nullptr;               // their sums, [kNLayer][512]
     int64_t step = 0;
+    // the launches' arguments over the batch buffers (plan_batch)
+    umma::ChainArgs fwd, bwd;
+    umma::ChainMaps fwd_maps, bwd_maps;
+    umma::DwArgs dw;
+    umma::DwMaps dw_maps;
     // batch buffers
     int B = 0;
-    bf16 *X = nullptr, *XT = nullptr, *H[3] = {}, *HT[3] = {}, *G[3] = {}, *GT[3] = {}, *dO = nullptr, *dOT = nullptr;
-    float *OUT = nullptr, *Y = nullptr, *loss = nullptr;
+    bf16 *X = nullptr, *H[3] = {}, *G[3] = {}, *dO = nullptr;
+    uint32_t *mask[3] = {};               // nonzero bits of the hidden activations, [B][16]
+    float *OUT = nullptr, *Y = nullptr;
+    float *loss = nullptr;                // one allocation with err: read back in one copy
     int64_t *idx = nullptr;
     // training set
     int64_t nset = 0;
@@ -472,59 +478,6 @@ struct bg_mlp {
 };
 
 namespace {
-
-int ensure_batch(bg_mlp *h, int B) {
-    if (B == h->B) return BG_OK;
-    // the batch buffers move: a captured training step holds their addresses
-    if (h->step_graph) {
-        cudaStreamSynchronize(h->stream);
-        cudaGraphExecDestroy(h->step_graph);
-        h->step_graph = nullptr;
-        h->graph_batch = 0;
-    }
-    int rc = 0;
-    if ((rc = dalloc(&h->X, (size_t)B * kIn))) return rc;
-    if ((rc = dalloc(&h->XT, (size_t)B * kIn))) return rc;
-    for (int l = 0; l < 3; ++l) {
-        if ((rc = dalloc(&h->H[l], (size_t)B * kHid))) return rc;
-        if ((rc = dalloc(&h->HT[l], (size_t)B * kHid))) return rc;
-        if ((rc = dalloc(&h->G[l], (size_t)B * kHid))) return rc;
-        if ((rc = dalloc(&h->GT[l], (size_t)B * kHid))) return rc;
-    }
-    if ((rc = dalloc(&h->dO, (size_t)B * kOutPad))) return rc;
-    if ((rc = dalloc(&h->dOT, (size_t)B * kOutPad))) return rc;
-    if ((rc = dalloc(&h->OUT, (size_t)B * kOutPad))) return rc;
-    if ((rc = dalloc(&h->Y, (size_t)B * h->ydim))) return rc;
-    if ((rc = dalloc(&h->idx, (size_t)B))) return rc;
-    for (int l = 0; l < kNLayer; ++l)
-        if ((rc = dalloc(&h->cs[l], (size_t)((B + 31) / 32) * kHid))) return rc;
-    if (!h->gbias && (rc = dalloc(&h->gbias, (size_t)kNLayer * kHid))) return rc;
-    h->B = B;
-    return BG_OK;
-}
-
-// forward of the batch in h->X -> h->OUT
-int forward(bg_mlp *h, int B) {
-    const bf16 *in = h->X;
-    int K = kIn;
-    for (int l = 0; l < 3; ++l) {
-        umma::GemmArgs g = gemm_args(in, K, h->Wb[l], K, B, kHid, K, h->err);
-        g.bias = h->b[l];
-        g.H = h->H[l];
-        g.ldh = kHid;
-        g.HT = h->HT[l];
-        g.ldht = B;
-        int rc = launch_gemm<kNT, umma::EPI_RELU_BF16>(g, 1, h->stream);
-        if (rc) return rc;
-        in = h->H[l];
-        K = kHid;
-    }
-    umma::GemmArgs g = gemm_args(in, kHid, h->Wb[3], kHid, B, kOutPad, kHid, h->err);
-    g.bias = h->b[3];
-    g.C = h->OUT;
-    g.ldc = kOutPad;
-    return launch_gemm<64, umma::EPI_BIAS_F32>(g, 1, h->stream);
-}
 
 // Bias-gradient partials of layer l: per-block column sums written by the
 // loss kernel (output layer, blocks of 256 rows, 64 columns) or by the
@@ -540,67 +493,126 @@ void bias_partials(const bg_mlp *h, int l, int B, const float **p, int *nblk, in
     }
 }
 
-// the bias gradients' sums (k_bias_reduce) for Adam and the flat gradient
-int reduce_bias(bg_mlp *h, int B, bool pdl) {
-    BiasRed r;
-    memset(&r, 0, sizeof r);
+// Arguments and tensor maps of the chains and the weight gradients over batch
+// buffers of B rows (a multiple of 128).
+int plan_batch(bg_mlp *h, int B) {
+    memset(&h->fwd, 0, sizeof h->fwd);
+    memset(&h->bwd, 0, sizeof h->bwd);
+    memset(&h->dw, 0, sizeof h->dw);
+    h->fwd.layers = kNLayer;
+    h->bwd.layers = kNLayer - 1;
+    h->fwd.rows = h->bwd.rows = B;
+    h->fwd.err = h->bwd.err = h->dw.err = h->err;
+    bool ok = tile_map(&h->fwd_maps.in, h->X, B, kIn, kIn, umma::kM, true) &&
+              tile_map(&h->bwd_maps.in, h->dO, B, kOutPad, kOutPad, umma::kM, true);
     for (int l = 0; l < kNLayer; ++l) {
-        bias_partials(h, l, B, &r.p[l], &r.nblk[l], &r.ld[l]);
-        r.rows[l] = h->rows[l];
-        r.blk0[l + 1] = r.blk0[l] + (r.rows[l] + 31) / 32;
+        umma::ChainLayer &L = h->fwd.L[l];
+        L.K = h->cols[l];
+        L.N = h->rows[l];
+        L.bias = h->b[l];
+        if (l < 3) {
+            L.keep = 1;
+            L.mask = h->mask[l];
+            ok = ok && tile_map(&h->fwd_maps.out[l], h->H[l], B, kHid, kHid, umma::kM, true);
+        } else {
+            L.C = h->OUT;
+        }
+        ok = ok && tile_map(&h->fwd_maps.w[l], h->Wb[l], L.N, L.K, L.K, std::min(L.N, umma::kChainN), true);
     }
-    r.out = h->gbias;
-    const dim3 grid((unsigned)r.blk0[kNLayer]), block(256);
-    if (pdl) MCK(launch_pdl(k_bias_reduce, grid, block, 0, h->stream, r));
-    else k_bias_reduce<<<grid, block, 0, h->stream>>>(r);
-    MCK(cudaGetLastError());
+    for (int q = 0; q < kNLayer - 1; ++q) {
+        const int l = 3 - q;                 // through W_l into hidden layer l - 1
+        umma::ChainLayer &L = h->bwd.L[q];
+        L.K = h->rows[l];
+        L.N = h->cols[l];
+        L.keep = 1;
+        L.mask = h->mask[l - 1];
+        L.colsum = h->cs[l - 1];
+        ok = ok && tile_map(&h->bwd_maps.out[q], h->G[l - 1], B, kHid, kHid, umma::kM, true);
+        ok = ok && tile_map(&h->bwd_maps.w[q], h->WbT[l], L.N, L.K, L.K, umma::kChainN, true);
+    }
+    // the weight gradients need whole 64-row chunks in each split (the training
+    // calls ask for it; the buffers of a forward call may have any 128 rows)
+    if (B % (kSplits * umma::kKc) == 0) {
+        h->dw.splits = kSplits;
+        h->dw.nk = B / kSplits / umma::kKc;
+        const int order[kNLayer] = {2, 1, 3, 0};             // the widest units first
+        for (int q = 0; q < kNLayer; ++q) {
+            const int l = order[q];
+            umma::DwProduct &p = h->dw.p[q];
+            p.M = h->rows[l];
+            p.N = h->cols[l];
+            p.nt = p.N == kHid ? umma::kDwN : 64;
+            p.tiles_m = (p.M + umma::kM - 1) / umma::kM;
+            p.tiles_n = p.N / p.nt;
+            p.unit0 = h->dw.units;
+            h->dw.units += p.tiles_m * p.tiles_n * kSplits;
+            p.C = h->gWl[l];
+            p.split_stride = (long long)p.M * p.N;
+            ok = ok && tile_map(&h->dw_maps.a[q], l == 3 ? h->dO : h->G[l], B, p.M, p.M, umma::kKc, true);
+            ok = ok && tile_map(&h->dw_maps.b[q], l > 0 ? h->H[l - 1] : h->X, B, p.N, p.N, umma::kKc, true);
+        }
+        umma::BiasRed &r = h->dw.bias;
+        for (int l = 0; l < kNLayer; ++l) {
+            bias_partials(h, l, B, &r.p[l], &r.nblk[l], &r.ld[l]);
+            r.rows[l] = h->rows[l];
+            r.blk0[l + 1] = r.blk0[l] + (r.rows[l] + 31) / 32;
+        }
+        r.out = h->gbias;
+    }
+    return ok ? BG_OK : fail(BG_ECUDA, "mlp: tensor map");
+}
+
+int ensure_batch(bg_mlp *h, int B) {
+    if (B == h->B) return BG_OK;
+    // the batch buffers move: a captured training step holds their addresses
+    if (h->step_graph) {
+        cudaStreamSynchronize(h->stream);
+        cudaGraphExecDestroy(h->step_graph);
+        h->step_graph = nullptr;
+        h->graph_batch = 0;
+    }
+    int rc = 0;
+    h->B = 0;
+    if ((rc = dalloc(&h->X, (size_t)B * kIn))) return rc;
+    for (int l = 0; l < 3; ++l) {
+        if ((rc = dalloc(&h->H[l], (size_t)B * kHid))) return rc;
+        if ((rc = dalloc(&h->G[l], (size_t)B * kHid))) return rc;
+        if ((rc = dalloc(&h->mask[l], (size_t)B * (kHid / 32)))) return rc;
+    }
+    if ((rc = dalloc(&h->dO, (size_t)B * kOutPad))) return rc;
+    if ((rc = dalloc(&h->OUT, (size_t)B * kOutPad))) return rc;
+    if ((rc = dalloc(&h->Y, (size_t)B * h->ydim))) return rc;
+    if ((rc = dalloc(&h->idx, (size_t)B))) return rc;
+    for (int l = 0; l < kNLayer; ++l)
+        if ((rc = dalloc(&h->cs[l], (size_t)((B + 31) / 32) * kHid))) return rc;
+    if (!h->gbias && (rc = dalloc(&h->gbias, (size_t)kNLayer * kHid))) return rc;
+    if ((rc = plan_batch(h, B))) return rc;
+    MCK(cudaStreamSynchronize(nullptr));     // the buffers are cleared before h->stream writes them
+    h->B = B;
     return BG_OK;
 }
 
-// backward from the loss gradient in h->dO / h->dOT: weight gradients of
-// layer l into its region of h->gW (kSplits partial slices over the batch),
-// bias gradients as the column-sum partials, and the input gradient of every
-// hidden layer (read against the weights before any update)
-int backward(bg_mlp *h, int B) {
-    int rc = 0;
-    const int splits = kSplits;
-    const int kper = B / splits;
-    const bf16 *gin = h->dO;
-    const bf16 *ginT = h->dOT;
-    int gK = kOutPad;
-    for (int l = 3; l >= 0; --l) {
-        // dW_l = gin^T . input_l   (input_l = H[l-1] or X)
-        const bf16 *inT = l > 0 ? h->HT[l - 1] : h->XT;
-        const int nin = l > 0 ? kHid : kIn;
-        {
-            umma::GemmArgs g = gemm_args(ginT, B, inT, B, h->rows[l], nin, B, h->err);
-            g.k_per_split = kper;
-            g.C = h->gWl[l];
-            g.ldc = nin;
-            g.split_stride = (int64_t)h->rows[l] * h->cols[l];
-            if (nin == kIn) rc = launch_gemm<64, umma::EPI_F32>(g, splits, h->stream);
-            else rc = launch_gemm<kNT, umma::EPI_F32>(g, splits, h->stream);
-            if (rc) return rc;
-        }
-        // gradient into the previous hidden layer; its epilogue also sums the
-        // columns for layer l-1's bias
-        if (l > 0) {
-            umma::GemmArgs g = gemm_args(gin, gK, h->WbT[l], h->rows[l], B, kHid, gK, h->err);
-            g.act = h->H[l - 1];
-            g.ldact = kHid;
-            g.H = h->G[l - 1];
-            g.ldh = kHid;
-            g.HT = h->GT[l - 1];
-            g.ldht = B;
-            g.colsum = h->cs[l - 1];
-            g.colsum_ld = kHid;
-            if ((rc = launch_gemm<kNT, umma::EPI_DRELU_BF16>(g, 1, h->stream))) return rc;
-            gin = h->G[l - 1];
-            ginT = h->GT[l - 1];
-            gK = kHid;
-        }
+// forward of the batch in h->X -> h->OUT, and (keep) the hidden activations -> h->H
+int forward(bg_mlp *h, bool keep) {
+    umma::ChainArgs g = h->fwd;
+    if (!keep)
+        for (int l = 0; l < 3; ++l) { g.L[l].keep = 0; g.L[l].mask = nullptr; }
+    return launch_chain<false>(g, h->fwd_maps, h->stream);
+}
+
+// backward from the loss gradient in h->dO: the hidden layers' gradients -> h->G
+// with the column-sum partials of their bias gradients, then the weight gradients'
+// partial slices -> h->gWl and the bias gradients -> h->gbias.  `advance`: also
+// count the training step.
+int backward(bg_mlp *h, bool advance) {
+    int rc = launch_chain<true>(h->bwd, h->bwd_maps, h->stream);
+    if (rc) return rc;
+    umma::DwArgs g = h->dw;
+    if (advance) {
+        g.batch_index = (long long *)h->dBatchIdx;
+        g.opt_step = (long long *)h->dOptStep;
     }
-    return BG_OK;
+    return launch_weight_gradients(g, h->dw_maps, h->stream);
 }
 
 // Adam's tensor descriptors: gradients from the partial slices of a batch
@@ -619,12 +631,14 @@ AdamAll adam_desc(bg_mlp *h, int B, float lr, const float *flat, float scale) {
         off += (int64_t)h->rows[l] * h->cols[l];
         AdamSeg &bb = a.seg[2 * l + 1];
         bb.P = h->b[l]; bb.m = h->mb[l]; bb.v = h->vb[l];
-        bb.grad = h->gbias + (int64_t)l * kHid; bb.splits = 1; bb.split_stride = 0;   // k_bias_reduce's sums
+        bb.grad = h->gbias + (int64_t)l * kHid; bb.splits = 1; bb.split_stride = 0;   // the weight-gradient kernel's sums
         bb.rows = h->rows[l]; bb.cols = 1; bb.rows_train = rows_train;
         a.off[2 * l + 1] = off;
         off += h->rows[l];
     }
     a.off[2 * kNLayer] = off;
+    for (int k = 0; k < 2 * kNLayer; ++k)
+        a.blk0[k + 1] = a.blk0[k] + (a.seg[k].Pb ? (a.seg[k].rows / 32) * (a.seg[k].cols / 32) : (a.seg[k].rows + 255) / 256);
     a.step = h->dOptStep;
     a.lr = lr; a.b1 = 0.9f; a.b2 = 0.999f; a.eps = 1e-8f; a.scale = scale;
     if (flat)
@@ -635,30 +649,31 @@ AdamAll adam_desc(bg_mlp *h, int B, float lr, const float *flat, float scale) {
 // Adam on every tensor in one launch (the step count is read on the device)
 int adam_all(bg_mlp *h, int B, float lr, const float *flat = nullptr, float scale = 1.f) {
     const AdamAll a = adam_desc(h, B, lr, flat, scale);
-    const int64_t off = a.off[2 * kNLayer];
-    MCK(launch_pdl(k_adam_all, dim3((unsigned)((off + 255) / 256)), dim3(256), 0, h->stream, a));
-    int tiles = 0;
-    for (int k = 0; k < 2 * kNLayer; ++k)
-        if (a.seg[k].PbT) tiles += ((a.seg[k].rows + 31) / 32) * ((a.seg[k].cols + 31) / 32);
-    if (tiles) MCK(launch_pdl(k_transpose_all, dim3((unsigned)tiles), dim3(32, 8), 0, h->stream, a));
+    MCK(launch_pdl(k_adam_all, dim3((unsigned)a.blk0[2 * kNLayer]), dim3(256), 0, h->stream, a));
+    return BG_OK;
+}
+
+int gather(bg_mlp *h, const int64_t *order, const int64_t *batch_index) {
+    MCK(launch_pdl(k_gather, dim3((unsigned)((h->B + 31) / 32)), dim3(256), 0, h->stream, (const float *)h->Xall,
+                   (const float *)h->Yall, order, batch_index, h->B, h->ydim, h->X, h->Y));
+    return BG_OK;
+}
+
+int loss_gradient(bg_mlp *h) {
+    MCK(launch_pdl(k_nll, dim3((h->B + 255) / 256), dim3(256), 0, h->stream, (const float *)h->OUT, (const float *)h->Y, h->B,
+                   h->ydim, h->dO, h->cs[kNLayer - 1], h->loss));
     return BG_OK;
 }
 
 // one training step on batch `*dBatchIdx` of h->perm: gather, forward, loss,
 // backward, Adam, counters
 int train_step(bg_mlp *h, int B, float lr) {
-    k_gather_at<<<B, 64, 0, h->stream>>>(h->Xall, h->Yall, h->perm, h->dBatchIdx, B, h->ydim, h->X, h->XT, h->Y);
-    int rc = forward(h, B);
-    if (rc) return rc;
-    MCK(launch_pdl(k_nll, dim3((B + 255) / 256), dim3(256), 0, h->stream, (const float *)h->OUT, (const float *)h->Y, B,
-                   h->ydim, h->dO, h->dOT, h->cs[kNLayer - 1], h->loss));
-    if ((rc = backward(h, B))) return rc;
-    if ((rc = reduce_bias(h, B, true))) return rc;
+    int rc = gather(h, h->perm, h->dBatchIdx);
+    if (rc || (rc = forward(h, true))) return rc;
+    if ((rc = loss_gradient(h))) return rc;
     // Adam's step count t is the step being taken (1 for the first)
-    MCK(launch_pdl(k_step_advance, dim3(1), dim3(1), 0, h->stream, h->dBatchIdx, h->dOptStep));
-    if ((rc = adam_all(h, B, lr))) return rc;
-    MCK(cudaGetLastError());
-    return BG_OK;
+    if ((rc = backward(h, true))) return rc;
+    return adam_all(h, B, lr);
 }
 
 // the epoch order buffers and the sort's scratch, kept for later calls
@@ -705,7 +720,6 @@ BG_API int bg_mlp_create(bg_mlp **out, int device, int ydim) {
     h->ydim = ydim;
     int rc = 0;
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) rc = fail(BG_ECUDA, "mlp: stream");
-    if (!rc) rc = dalloc(&h->err, 1);
     for (int l = 0; l < kNLayer && !rc; ++l) {
         const size_t n = (size_t)h->rows[l] * h->cols[l];
         if (!rc) rc = dalloc(&h->W[l], n);
@@ -720,14 +734,14 @@ BG_API int bg_mlp_create(bg_mlp **out, int device, int ydim) {
     {
         size_t tot = 0;
         for (int l = 0; l < kNLayer; ++l) tot += (size_t)kSplits * h->rows[l] * h->cols[l];
-        tot = std::max(tot, (size_t)kSplits * kHid * kHid);
         if (!rc) rc = dalloc(&h->gW, tot);
         size_t o = 0;
         for (int l = 0; l < kNLayer && !rc; ++l) { h->gWl[l] = h->gW + o; o += (size_t)kSplits * h->rows[l] * h->cols[l]; }
     }
     if (!rc) rc = dalloc(&h->dBatchIdx, 1);
     if (!rc) rc = dalloc(&h->dOptStep, 1);
-    if (!rc) rc = dalloc(&h->loss, 1);
+    if (!rc) rc = dalloc(&h->loss, 2);
+    if (!rc) h->err = reinterpret_cast<int *>(h->loss + 1);
     if (rc) {
         bg_mlp_destroy(h);
         return rc;
@@ -744,10 +758,10 @@ BG_API int bg_mlp_destroy(bg_mlp *h) {
         dfree(h->W[l]); dfree(h->b[l]); dfree(h->mW[l]); dfree(h->vW[l]); dfree(h->mb[l]); dfree(h->vb[l]);
         dfree(h->Wb[l]); dfree(h->WbT[l]);
     }
-    for (int l = 0; l < 3; ++l) { dfree(h->H[l]); dfree(h->HT[l]); dfree(h->G[l]); dfree(h->GT[l]); }
-    dfree(h->X); dfree(h->XT); dfree(h->dO); dfree(h->dOT); dfree(h->OUT); dfree(h->Y); dfree(h->idx);
+    for (int l = 0; l < 3; ++l) { dfree(h->H[l]); dfree(h->G[l]); dfree(h->mask[l]); }
+    dfree(h->X); dfree(h->dO); dfree(h->OUT); dfree(h->Y); dfree(h->idx);
     for (int l = 0; l < kNLayer; ++l) dfree(h->cs[l]);
-    dfree(h->gW); dfree(h->gflat); dfree(h->loss); dfree(h->err); dfree(h->Xall); dfree(h->Yall);
+    dfree(h->gW); dfree(h->gflat); dfree(h->loss); dfree(h->Xall); dfree(h->Yall);
     dfree(h->dBatchIdx); dfree(h->dOptStep); dfree(h->pkeys); dfree(h->pkeys_out); dfree(h->pvals); dfree(h->perm);
     if (h->sort_tmp) cudaFree(h->sort_tmp);
     if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
@@ -791,20 +805,15 @@ BG_API int bg_mlp_forward(bg_mlp *h, const float *X, int64_t n, float *out) {
     const int B = (int)((n + 127) / 128 * 128);
     int rc = ensure_batch(h, B);
     if (rc) return rc;
-    std::vector<bf16> xb((size_t)B * kIn, __float2bfloat16_rn(0.f)), xt((size_t)B * kIn, __float2bfloat16_rn(0.f));
+    std::vector<bf16> xb((size_t)B * kIn, __float2bfloat16_rn(0.f));
     for (int64_t r = 0; r < n; ++r)
-        for (int j = 0; j < kIn; ++j) {
-            const bf16 v = __float2bfloat16_rn(X[r * kIn + j]);
-            xb[(size_t)r * kIn + j] = v;
-            xt[(size_t)j * B + r] = v;
-        }
+        for (int j = 0; j < kIn; ++j) xb[(size_t)r * kIn + j] = __float2bfloat16_rn(X[r * kIn + j]);
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, h->stream);
     MCK(cudaMemcpyAsync(h->X, xb.data(), xb.size() * sizeof(bf16), cudaMemcpyHostToDevice, h->stream));
-    MCK(cudaMemcpyAsync(h->XT, xt.data(), xt.size() * sizeof(bf16), cudaMemcpyHostToDevice, h->stream));
-    if ((rc = forward(h, B))) return rc;
+    if ((rc = forward(h, false))) return rc;
     std::vector<float> o((size_t)B * kOutPad);
     MCK(cudaMemcpyAsync(o.data(), h->OUT, o.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     cudaEventRecord(e1, h->stream);
@@ -927,20 +936,19 @@ BG_API int bg_mlp_step_gradients(bg_mlp *h, int batch, int64_t row0, float *loss
     const int64_t bidx = row0 / batch;
     MCK(cudaMemcpyAsync(h->dBatchIdx, &bidx, sizeof(int64_t), cudaMemcpyHostToDevice, h->stream));
     MCK(cudaMemsetAsync(h->loss, 0, sizeof(float), h->stream));
-    k_gather_at<<<batch, 64, 0, h->stream>>>(h->Xall, h->Yall, h->perm, h->dBatchIdx, batch, h->ydim, h->X, h->XT, h->Y);
-    if ((rc = forward(h, batch))) return rc;
-    k_nll<<<(batch + 255) / 256, 256, 0, h->stream>>>(h->OUT, h->Y, batch, h->ydim, h->dO, h->dOT,
-                                                       h->cs[kNLayer - 1], h->loss);
-    if ((rc = backward(h, batch))) return rc;
-    if ((rc = reduce_bias(h, batch, false))) return rc;
+    if ((rc = gather(h, h->perm, h->dBatchIdx)) || (rc = forward(h, true)) || (rc = loss_gradient(h)) ||
+        (rc = backward(h, false)))
+        return rc;
     const AdamAll a = adam_desc(h, batch, 0.f, nullptr, 1.f);
     k_grad_flat<<<(unsigned)((nflat + 255) / 256), 256, 0, h->stream>>>(a, h->gflat);
     MCK(cudaGetLastError());
-    float ls = 0;
-    MCK(cudaMemcpyAsync(&ls, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    float out[2];                        // the loss and the error flag
+    MCK(cudaMemcpyAsync(out, h->loss, sizeof out, cudaMemcpyDeviceToHost, h->stream));
     MCK(cudaStreamSynchronize(h->stream));
-    if ((rc = check_err(h))) return rc;
-    if (loss) *loss = ls;
+    int e;
+    memcpy(&e, &out[1], sizeof e);
+    if (e) return fail(BG_ETIMEOUT, "mlp: a tensor-core wait gave up");
+    if (loss) *loss = out[0];
     if (grad) *grad = h->gflat;
     if (ngrad) *ngrad = nflat;
     return BG_OK;
@@ -970,35 +978,18 @@ BG_API int bg_mlp_gradients(bg_mlp *h, int batch, float *loss, float *const *dW,
     for (int i = 0; i < batch; ++i) idx[i] = i;
     MCK(cudaMemcpyAsync(h->idx, idx.data(), batch * sizeof(int64_t), cudaMemcpyHostToDevice, h->stream));
     MCK(cudaMemsetAsync(h->loss, 0, sizeof(float), h->stream));
-    k_gather<<<batch, 64, 0, h->stream>>>(h->Xall, h->Yall, h->idx, batch, h->ydim, h->X, h->XT, h->Y);
-    if ((rc = forward(h, batch))) return rc;
-    k_nll<<<(batch + 255) / 256, 256, 0, h->stream>>>(h->OUT, h->Y, batch, h->ydim, h->dO, h->dOT,
-                                                       h->cs[kNLayer - 1], h->loss);
-    // run the backward pass layer by layer, reading each layer's gradient
-    // before the next layer reuses the scratch
+    if ((rc = gather(h, h->idx, nullptr)) || (rc = forward(h, true)) || (rc = loss_gradient(h)) || (rc = backward(h, false)))
+        return rc;
     const int splits = kSplits;
-    const int kper = batch / splits;
-    const bf16 *gin = h->dO, *ginT = h->dOT;
-    int gK = kOutPad;
     for (int l = 3; l >= 0; --l) {
-        const bf16 *inT = l > 0 ? h->HT[l - 1] : h->XT;
-        const int nin = l > 0 ? kHid : kIn;
-        umma::GemmArgs g = gemm_args(ginT, batch, inT, batch, h->rows[l], nin, batch, h->err);
-        g.k_per_split = kper;
-        g.C = h->gW;
-        g.ldc = nin;
-        g.split_stride = (int64_t)kHid * kHid;
-        rc = nin == kIn ? launch_gemm<64, umma::EPI_F32>(g, splits, h->stream)
-                        : launch_gemm<kNT, umma::EPI_F32>(g, splits, h->stream);
-        if (rc) return rc;
-        std::vector<float> part((size_t)splits * kHid * kHid);
-        MCK(cudaMemcpyAsync(part.data(), h->gW, part.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        const size_t n = (size_t)h->rows[l] * h->cols[l];
+        std::vector<float> part((size_t)splits * n);
+        MCK(cudaMemcpyAsync(part.data(), h->gWl[l], part.size() * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
         MCK(cudaStreamSynchronize(h->stream));
-        const size_t n = (size_t)h->rows[l] * nin;
         if (dW && dW[l])
             for (size_t i = 0; i < n; ++i) {
                 float s = 0;
-                for (int z = 0; z < splits; ++z) s += part[(size_t)z * kHid * kHid + i];
+                for (int z = 0; z < splits; ++z) s += part[(size_t)z * n + i];
                 dW[l][i] = s;
             }
         if (db && db[l]) {
@@ -1013,21 +1004,6 @@ BG_API int bg_mlp_gradients(bg_mlp *h, int batch, float *loss, float *const *dW,
                 for (int z = 0; z < nblk; ++z) s += r < ld ? cp[(size_t)z * ld + r] : 0.f;
                 db[l][r] = s;
             }
-        }
-        if (l > 0) {
-            umma::GemmArgs g2 = gemm_args(gin, gK, h->WbT[l], h->rows[l], batch, kHid, gK, h->err);
-            g2.act = h->H[l - 1];
-            g2.ldact = kHid;
-            g2.H = h->G[l - 1];
-            g2.ldh = kHid;
-            g2.HT = h->GT[l - 1];
-            g2.ldht = batch;
-            g2.colsum = h->cs[l - 1];
-            g2.colsum_ld = kHid;
-            if ((rc = launch_gemm<kNT, umma::EPI_DRELU_BF16>(g2, 1, h->stream))) return rc;
-            gin = h->G[l - 1];
-            ginT = h->GT[l - 1];
-            gK = kHid;
         }
     }
     if (loss) MCK(cudaMemcpy(loss, h->loss, sizeof(float), cudaMemcpyDeviceToHost));
@@ -1051,7 +1027,7 @@ BG_API int bg_gemm_bf16(int64_t M, int64_t N, int64_t K, const void *A, const vo
     umma::GemmArgs g = gemm_args((const bf16 *)A, (int)K, (const bf16 *)B, (int)K, (int)M, (int)N, (int)K, err);
     g.C = C;
     g.ldc = (int)N;
-    int rc = launch_gemm<128, umma::EPI_F32>(g, 1, st);
+    int rc = launch_gemm<128>(g, 1, st);
     cudaError_t e = cudaStreamSynchronize(st);
     int ev = 0;
     cudaMemcpy(&ev, err, sizeof(int), cudaMemcpyDeviceToHost);

@@ -13,13 +13,9 @@
 // four tcgen05.mma (K = 16 each) per chunk and commits them to the chunk's
 // mbarrier; a stage is refilled only after that mbarrier completes.  The
 // accumulator lives in TMEM (lane = tile row, one column per output column)
-// and is read back by every warp for its 32 rows with tcgen05.ld; the
-// epilogue is fused (bias, ReLU, ReLU gradient, transposed copies, column
-// sums).  Row-major results go through the idle stage buffers: each warp
-// stages its 32 x NT block in shared memory and writes whole rows with
-// 16-byte stores; the ReLU mask of the gradient epilogue is read the same
-// way.  Transposed copies are written from registers (32 consecutive rows
-// of one column per warp store).
+// and is read back by every warp for its 32 rows with tcgen05.ld.  Results go
+// through the idle stage buffers: each warp stages its 32 x NT block in shared
+// memory and writes whole rows with 16-byte stores.
 //
 // With TMA (template flag, when the operands' rows are 16-byte aligned) the
 // stages are filled by cp.async.bulk.tensor from 2-D tensor maps (K inner,
@@ -51,13 +47,6 @@ constexpr uint32_t kLBO = 128;   // bytes between core matrices along K
 constexpr uint32_t kSBO = 1024;  // bytes between 8-row groups
 constexpr long long kSpinLimit = 1ll << 24;
 
-enum Epi : int {
-    EPI_F32 = 0,        // C fp32 (optionally per split), no bias
-    EPI_BIAS_F32 = 1,   // C fp32 = acc + bias[n]
-    EPI_RELU_BF16 = 2,  // H bf16 = relu(acc + bias[n]), and H^T
-    EPI_DRELU_BF16 = 3  // G bf16 = acc * (act[m][n] > 0), and G^T
-};
-
 struct GemmArgs {
     const __nv_bfloat16 *A;   // [M][lda]
     const __nv_bfloat16 *B;   // [N][ldb]
@@ -66,16 +55,6 @@ struct GemmArgs {
     float *C;                 // fp32 out [split][M][ldc]
     int ldc;
     long long split_stride;   // elements between split slices of C
-    const float *bias;        // [N] or null
-    __nv_bfloat16 *H;         // bf16 out [M][ldh]
-    int ldh;
-    __nv_bfloat16 *HT;        // bf16 transposed out [N][ldht] or null
-    int ldht;
-    const __nv_bfloat16 *act; // [M][ldact] for EPI_DRELU_BF16
-    int ldact;
-    int n_valid;              // columns >= n_valid are written as 0 (bf16 outs) / skipped (fp32)
-    float *colsum;            // EPI_DRELU_BF16: column sums of the bf16 result over each 32-row
-    int colsum_ld;            //   quarter of a row tile, at colsum[(4 * row tile + quarter) * colsum_ld + col] (or null)
     int *err;                 // error flag (device)
 };
 
@@ -107,6 +86,21 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return d;
 }
 
+// MN-major tile (the K index is the memory row) in the 128-byte swizzled
+// layout: 64 consecutive M or N elements of one K are a 128-byte line, 8 lines
+// an atom (stride byte offset between atoms along K: 1024), the next 64
+// elements a whole box of kKc lines on (leading byte offset).  The K-step of
+// one MMA (16 lines) advances the start address by 2048 bytes.
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+    d |= (uint64_t)(((uint32_t)kKc * 128u) >> 4) << 16;
+    d |= (uint64_t)(1024u >> 4) << 32;
+    d |= (uint64_t)1 << 46;                          // sm100 descriptor version
+    d |= (uint64_t)2 << 61;                          // layout: 128-byte swizzle
+    return d;
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -119,9 +113,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map
         : "memory");
 }
 
-// kind::f16 instruction descriptor: D f32, A bf16, B bf16, both K-major.
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// kind::f16 instruction descriptor: D f32, A bf16, B bf16, both K-major or (mn)
+// both MN-major.
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N, bool mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (mn ? (1u << 15) | (1u << 16) : 0u) | ((uint32_t)(N >> 3) << 17) |
+           ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ uint32_t tile_off(int r, int q) {
@@ -200,7 +196,6 @@ struct Smem {
     alignas(8) unsigned long long bar[kStages];   // stage consumed (MMAs committed)
     alignas(8) unsigned long long full[kStages];  // stage filled (TMA path)
     alignas(8) unsigned long long done;           // every MMA finished (TMA path)
-    float bias[NT];
     uint32_t tmem_base;
     int failed;
 };
@@ -229,7 +224,7 @@ __device__ __forceinline__ void load_stage(Smem<NT> &sm, int st, const GemmArgs 
     }
 }
 
-template <int NT, int EPI, bool TMA>
+template <int NT, bool TMA>
 __global__ void __launch_bounds__(kThreads, 1) k_gemm(const GemmArgs g, const __grid_constant__ CUtensorMap ta,
                                                       const __grid_constant__ CUtensorMap tb) {
     extern __shared__ unsigned char smem_raw[];
@@ -242,8 +237,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const GemmArgs g, const __
     const int kend = min(g.K, kbeg + g.k_per_split);
     const int nk = (kend - kbeg) / kKc;
 
-    if ((EPI == EPI_RELU_BF16 || EPI == EPI_BIAS_F32) && tid < NT)
-        sm.bias[tid] = (n0 + tid < g.N) ? g.bias[n0 + tid] : 0.f;
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
             mbar_init(smem_u32(&sm.bar[s]), 1);
@@ -360,53 +353,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const GemmArgs g, const __
     if (sm.failed) {
         if (tid == 0 && g.err) atomicExch(g.err, 1);
     } else {
-        // epilogue: warp w owns tile rows 32w .. 32w+31, TMEM lanes alike
-        constexpr bool kBF = (EPI == EPI_RELU_BF16 || EPI == EPI_DRELU_BF16);
-        constexpr int kEsz = kBF ? 2 : 4;
-        constexpr int kRowE = NT + 16 / kEsz;                   // staged row: NT elements + 16 bytes
-        constexpr int kPieces = NT * kEsz / 16;                 // 16-byte pieces per row
-        static_assert(4 * 32 * kRowE * kEsz + 4 * NT * 4 <= sizeof(((Smem<NT> *)0)->a) +
-                                                             sizeof(((Smem<NT> *)0)->b),
+        // epilogue: warp w owns tile rows 32w .. 32w+31, TMEM lanes alike; its
+        // block goes through the idle stage buffers so that whole rows are
+        // written with 16-byte stores
+        constexpr int kRowE = NT + 4;                           // staged row: NT elements + 16 bytes
+        constexpr int kPieces = NT / 4;                         // 16-byte pieces per row
+        static_assert(4 * 32 * kRowE * 4 <= sizeof(((Smem<NT> *)0)->a) + sizeof(((Smem<NT> *)0)->b),
                       "epilogue staging exceeds the stage buffers");
-        unsigned char *stage = &sm.a[0][0] + (size_t)warp * 32 * kRowE * kEsz;
-        float *red = reinterpret_cast<float *>(&sm.a[0][0] + (size_t)4 * 32 * kRowE * kEsz);
+        float *stage = reinterpret_cast<float *>(&sm.a[0][0]) + (size_t)warp * 32 * kRowE;
         const int wrow0 = m0 + warp * 32;
-        const int row = wrow0 + lane;
-        const bool row_ok = row < g.M;
-        // row-major destination of this epilogue
-        unsigned char *dst = nullptr;
-        int ldo = 0, col_limit = g.N;
-        if (EPI == EPI_F32 || EPI == EPI_BIAS_F32) {
-            dst = reinterpret_cast<unsigned char *>(g.C + (long long)blockIdx.z * g.split_stride);
-            ldo = g.ldc;
-            col_limit = min(g.N, g.n_valid);
-        } else {
-            dst = reinterpret_cast<unsigned char *>(g.H);
-            ldo = g.ldh;
-        }
-        const bool vec_out = (((size_t)ldo * kEsz) % 16 == 0) && (((uintptr_t)dst & 15) == 0);
-        if (EPI == EPI_DRELU_BF16) {
-            // the mask source, rows of act, into the staging rows
-            const bool vec_in = (((size_t)g.ldact * 2) % 16 == 0) && (((uintptr_t)g.act & 15) == 0);
-            for (int p = lane; p < 32 * kPieces; p += 32) {
-                const int r = p / kPieces, q = p % kPieces;
-                const int grow = wrow0 + r, gcol = n0 + q * 8;
-                uint4 v = make_uint4(0, 0, 0, 0);
-                if (grow < g.M) {
-                    const __nv_bfloat16 *src = g.act + (long long)grow * g.ldact + gcol;
-                    if (vec_in && gcol + 8 <= g.N) {
-                        v = *reinterpret_cast<const uint4 *>(src);
-                    } else {
-                        __nv_bfloat16 t[8];
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) t[e] = gcol + e < g.N ? src[e] : __float2bfloat16_rn(0.f);
-                        v = *reinterpret_cast<uint4 *>(t);
-                    }
-                }
-                *reinterpret_cast<uint4 *>(stage + ((size_t)r * kRowE + q * 8) * 2) = v;
-            }
-            __syncwarp();
-        }
+        float *dst = g.C + (long long)blockIdx.z * g.split_stride;
+        const bool vec_out = (((size_t)g.ldc * 4) % 16 == 0) && (((uintptr_t)dst & 15) == 0);
 #pragma unroll 1
         for (int cb = 0; cb < NT; cb += 16) {
             float v[16];
@@ -416,73 +373,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm(const GemmArgs g, const __
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = 0.f;
             }
-            unsigned char *srow = stage + ((size_t)lane * kRowE + cb) * kEsz;
-            if (kBF) {
-                __nv_bfloat16 hv[16];
-                __nv_bfloat16 av[16];
-                if (EPI == EPI_DRELU_BF16) {
-                    *reinterpret_cast<uint4 *>(av) = *reinterpret_cast<const uint4 *>(srow);
-                    *reinterpret_cast<uint4 *>(av + 8) = *reinterpret_cast<const uint4 *>(srow + 16);
-                }
+            float *srow = stage + (size_t)lane * kRowE + cb;
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int col = n0 + cb + i;
-                    float x = v[i];
-                    if (EPI == EPI_RELU_BF16) {
-                        x = col < g.N ? x + sm.bias[cb + i] : 0.f;
-                        x = x > 0.f ? x : 0.f;
-                    } else {
-                        x = __bfloat162float(av[i]) > 0.f ? x : 0.f;
-                    }
-                    if (col >= g.n_valid || col >= g.N || !row_ok) x = 0.f;
-                    hv[i] = __float2bfloat16_rn(x);
-                    if (g.HT && row_ok && col < g.N) g.HT[(long long)col * g.ldht + row] = hv[i];
-                }
-                *reinterpret_cast<uint4 *>(srow) = *reinterpret_cast<uint4 *>(hv);
-                *reinterpret_cast<uint4 *>(srow + 16) = *reinterpret_cast<uint4 *>(hv + 8);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const int col = n0 + cb + i;
-                    if (EPI == EPI_BIAS_F32 && col < g.N) v[i] += sm.bias[cb + i];
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i += 4)
-                    *reinterpret_cast<float4 *>(srow + i * 4) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-            }
+            for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4 *>(srow + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
         }
         __syncwarp();
-        if (EPI == EPI_DRELU_BF16 && g.colsum) {
-            // column sums of the bf16 results over the CTA's rows, fixed order
-            for (int c = lane; c < NT; c += 32) {
-                float sum = 0.f;
-                for (int r = 0; r < 32; ++r)
-                    sum += __bfloat162float(*reinterpret_cast<const __nv_bfloat16 *>(stage + ((size_t)r * kRowE + c) * 2));
-                red[warp * NT + c] = sum;
-            }
-        }
-        // whole rows out with 16-byte stores
         for (int p = lane; p < 32 * kPieces; p += 32) {
             const int r = p / kPieces, q = p % kPieces;
-            const int grow = wrow0 + r;
+            const int grow = wrow0 + r, gcol = n0 + q * 4;
             if (grow >= g.M) continue;
-            constexpr int kPer = 16 / kEsz;
-            const int gcol = n0 + q * kPer;
-            const unsigned char *src = stage + ((size_t)r * kRowE + q * kPer) * kEsz;
-            unsigned char *d = dst + ((size_t)grow * ldo + gcol) * kEsz;
-            if (vec_out && gcol + kPer <= col_limit) {
-                *reinterpret_cast<uint4 *>(d) = *reinterpret_cast<const uint4 *>(src);
+            const float *src = stage + (size_t)r * kRowE + q * 4;
+            float *d = dst + (size_t)grow * g.ldc + gcol;
+            if (vec_out && gcol + 4 <= g.N) {
+                *reinterpret_cast<float4 *>(d) = *reinterpret_cast<const float4 *>(src);
             } else {
-                for (int e = 0; e < kPer && gcol + e < col_limit; ++e)
-                    for (int by = 0; by < kEsz; ++by) d[e * kEsz + by] = src[e * kEsz + by];
-            }
-        }
-        if (EPI == EPI_DRELU_BF16 && g.colsum) {
-            __syncwarp();
-            // this warp's 32-row column sums: row (4 blockIdx.x + warp) of colsum
-            for (int c = lane; c < NT; c += 32) {
-                const int col = n0 + c;
-                if (col < g.N) g.colsum[(long long)(4 * blockIdx.x + warp) * g.colsum_ld + col] = red[warp * NT + c];
+                for (int e = 0; e < 4 && gcol + e < g.N; ++e) d[e] = src[e];
             }
         }
     }
@@ -504,18 +409,17 @@ constexpr size_t smem_bytes() {
 // K-chunk instead of eight 16-byte-wide ones; 6-8 stages in flight).
 // A grid of at most one CTA per SM walks the output tiles (consecutive CTAs
 // take consecutive row tiles of one column tile, so they share the B tile in
-// L2).  Six warps per CTA:
+// L2).  Ten warps per CTA:
 //   warp 0  producer: one thread fills a PStages-deep ring of operand
 //           stages with TMA boxes (full[s] armed with the expected bytes,
 //           refilled after empty[s], which the MMAs of the stage commit to);
 //   warp 1  MMA: one thread issues the four tcgen05.mma of each K-chunk into
 //           one of two TMEM accumulators (2 x NT columns) and commits the
 //           finished tile to acc_full[buf];
-//   warps 2-5  epilogue: tcgen05.ld of their 32-lane quarter, the fused
-//           epilogue, stores straight from registers (each thread writes 16
-//           consecutive columns of its row: whole 32-byte sectors; the
-//           transposed copy is one 64-byte run per column and warp), then
-//           acc_empty[buf] frees the accumulator.
+//   warps 2-9  epilogue, two per 32-lane quarter: tcgen05.ld of half of the
+//           columns, then acc_empty[buf] frees the accumulator; stores
+//           straight from registers (each thread writes 16 consecutive columns
+//           of its row: whole 32-byte sectors).
 // So the epilogue of tile i runs while the MMAs of tile i+1 accumulate into
 // the other buffer, and TMEM allocation, barrier set-up and pipeline fill are
 // paid once per CTA instead of once per tile.  Every wait is bounded; a wait
@@ -543,7 +447,6 @@ struct PSmem {
     alignas(8) unsigned long long acc_full[2];
     alignas(8) unsigned long long acc_empty[2];
     alignas(8) unsigned long long done;
-    float red[4][NT];          // per-quarter column sums (EPI_DRELU_BF16)
     uint32_t tmem_base;
     int failed;
 };
@@ -565,92 +468,19 @@ __device__ __forceinline__ void tile_coords(int t, int tiles_m, int tiles_n, int
     z = r / tiles_n;
 }
 
-// The ReLU mask source of a DRELU epilogue, 16 columns of the thread's row
-// from c0 on (0 past the matrix), read before the accumulator is ready.
-__device__ __forceinline__ void p_load_act(const GemmArgs &g, int row, int c0, uint4 (&u)[2]) {
-    u[0] = make_uint4(0, 0, 0, 0);
-    u[1] = make_uint4(0, 0, 0, 0);
+// 16 accumulator columns of the thread's row to C
+__device__ __forceinline__ void p_store16(const GemmArgs &g, const float (&v)[16], int row, int c0, int z) {
     if (row >= g.M) return;
-    const __nv_bfloat16 *src = g.act + (long long)row * g.ldact + c0;
-    if (((((uintptr_t)src) & 15) == 0) && c0 + 16 <= g.N) {
-        u[0] = *reinterpret_cast<const uint4 *>(src);
-        u[1] = *reinterpret_cast<const uint4 *>(src + 8);
+    float *d = g.C + (long long)z * g.split_stride + (long long)row * g.ldc + c0;
+    if (((((uintptr_t)d) & 15) == 0) && c0 + 16 <= g.N) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4) reinterpret_cast<float4 *>(d)[i / 4] = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
     } else {
-        __nv_bfloat16 *h = reinterpret_cast<__nv_bfloat16 *>(u);
-        for (int i = 0; i < 16 && c0 + i < g.N; ++i) h[i] = src[i];
+        for (int i = 0; i < 16 && c0 + i < g.N; ++i) d[i] = v[i];
     }
 }
 
-template <int NT, int EPI>
-__device__ __forceinline__ void p_epilogue_chunk(const GemmArgs &g, const float (&v)[16], int row, int n0, int cb,
-                                                 int ntile_m, int quarter, int lane, PSmem<NT> &sm, int z,
-                                                 const uint4 (&actu)[2]) {
-    constexpr bool kBF = (EPI == EPI_RELU_BF16 || EPI == EPI_DRELU_BF16);
-    const bool row_ok = row < g.M;
-    const int c0 = n0 + cb;
-    if (kBF) {
-        __nv_bfloat16 hv[16];
-        float act[16];
-        if (EPI == EPI_DRELU_BF16) {
-            const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(actu);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) act[i] = __bfloat162float(h[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int col = c0 + i;
-            float x = v[i];
-            if (EPI == EPI_RELU_BF16) {
-                x = col < g.N ? x + __ldg(g.bias + col) : 0.f;
-                x = x > 0.f ? x : 0.f;
-            } else {
-                x = act[i] > 0.f ? x : 0.f;
-            }
-            if (col >= g.n_valid || col >= g.N || !row_ok) x = 0.f;
-            hv[i] = __float2bfloat16_rn(x);
-        }
-        if (row_ok) {
-            __nv_bfloat16 *d = g.H + (long long)row * g.ldh + c0;
-            if (((((uintptr_t)d) & 15) == 0) && c0 + 16 <= g.N) {
-                reinterpret_cast<uint4 *>(d)[0] = reinterpret_cast<const uint4 *>(hv)[0];
-                reinterpret_cast<uint4 *>(d)[1] = reinterpret_cast<const uint4 *>(hv)[1];
-            } else {
-                for (int i = 0; i < 16 && c0 + i < g.N; ++i) d[i] = hv[i];
-            }
-            if (g.HT)
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    if (c0 + i < g.N) g.HT[(long long)(c0 + i) * g.ldht + row] = hv[i];
-        }
-        if (EPI == EPI_DRELU_BF16 && g.colsum) {
-            // column sums of the bf16 results over the quarter's 32 rows
-            // (a fixed butterfly order, so the result is deterministic)
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float s = __bfloat162float(hv[i]);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                if (lane == 0) sm.red[quarter][cb + i] = s;
-            }
-        }
-    } else {
-        if (row_ok) {
-            const int limit = min(g.N, g.n_valid);
-            float o[16];
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o[i] = (EPI == EPI_BIAS_F32 && c0 + i < g.N) ? v[i] + __ldg(g.bias + c0 + i) : v[i];
-            float *d = g.C + (long long)z * g.split_stride + (long long)row * g.ldc + c0;
-            if (((((uintptr_t)d) & 15) == 0) && c0 + 16 <= limit) {
-#pragma unroll
-                for (int i = 0; i < 16; i += 4) reinterpret_cast<float4 *>(d)[i / 4] = make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-            } else {
-                for (int i = 0; i < 16 && c0 + i < limit; ++i) d[i] = o[i];
-            }
-        }
-    }
-}
-
-template <int NT, int EPI>
+template <int NT>
 __global__ void __launch_bounds__(kPThreads, 1) k_gemm_p(const GemmArgs g, const __grid_constant__ CUtensorMap ta,
                                                         const __grid_constant__ CUtensorMap tb, int tiles_m,
                                                         int tiles_n, int splits) {
@@ -765,11 +595,6 @@ __global__ void __launch_bounds__(kPThreads, 1) k_gemm_p(const GemmArgs g, const
             tile_coords(t, tiles_m, tiles_n, mt, nt, z);
             const int m0 = mt * kM, n0 = nt * NT;
             const int row = m0 + quarter * 32 + lane;
-            // the mask source is read while the MMAs of the tile run
-            uint4 actu[kQ][2];
-            if (EPI == EPI_DRELU_BF16)
-#pragma unroll
-                for (int q = 0; q < kQ; ++q) p_load_act(g, row, n0 + 16 * (half * kQ + q), actu[q]);
             bool ok = mbar_wait(smem_u32(&sm.acc_full[buf]), (uint32_t)(use & 1));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok || *(volatile int *)&sm.failed) { if (lane == 0) atomicExch(&sm.failed, 1); break; }
@@ -789,14 +614,7 @@ __global__ void __launch_bounds__(kPThreads, 1) k_gemm_p(const GemmArgs g, const
                 float v[16];
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(raw[q][i]);
-                p_epilogue_chunk<NT, EPI>(g, v, row, n0, 16 * (half * kQ + q), mt, quarter, lane, sm, z, actu[q]);
-            }
-            if (EPI == EPI_DRELU_BF16 && g.colsum) {
-                // this quarter's 32-row column sums: row (4 mt + quarter) of colsum
-                __syncwarp();
-                for (int c = half * (NT / 2) + lane; c < (half + 1) * (NT / 2); c += 32)
-                    if (n0 + c < g.N) g.colsum[(long long)(4 * mt + quarter) * g.colsum_ld + n0 + c] = sm.red[quarter][c];
-                __syncwarp();
+                p_store16(g, v, row, n0 + 16 * (half * kQ + q), z);
             }
         }
     }
