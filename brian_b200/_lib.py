@@ -101,6 +101,7 @@ ENGINE_ONLY = {
     "fit_evaluate": [_vp, _vp, _vp],
     "fit_features": [_vp, _vp],
     "fit_train_features": [_vp, _i64, _vp, _vp, _vp, _vp, _P(ct.c_float)],
+    "conn_read_weights": [_vp, _i32, _vp, _i64],
     "mlp_last_forward_ms": [_vp, _P(ct.c_float)],
     "spike_features": [ct.c_int, _i64, _vp, _vp, _vp, _vp, _i64, _dbl, _vp],
     "fit_set_blocks_per_sm": [_vp, _i32],
@@ -372,6 +373,16 @@ class Runtime(object):
     def conn_get_weights(self, cid, count):
         out = np.empty(count, dtype=np.float64)
         self._c(self.t.conn_get_weights(self.h, cid, _ptr(out)), "conn_get_weights")
+        return out
+
+    def conn_read_weights(self, cid, count, dtype):
+        """The weights in the connection's own type (conn_get_weights for a
+        table without the typed read)."""
+        read = getattr(self.t, "conn_read_weights", None)
+        if read is None or np.dtype(dtype) not in (np.float32, np.float64):
+            return self.conn_get_weights(cid, count).astype(dtype)
+        out = np.empty(count, dtype=dtype)
+        self._c(read(self.h, cid, _ptr(out), out.nbytes), "conn_read_weights")
         return out
 
     def conn_set_weights(self, cid, w):

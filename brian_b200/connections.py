@@ -416,7 +416,7 @@ class Connection(EngineBound):
 
     def _weights(self):
         if self._binding is not None:
-            self._w = self._binding.read_weights(self).astype(self.dtype)
+            self._w = self._binding.read_weights(self)
             self._wshared = None
         elif self._w is None and self._wshared is not None:
             self._w = np.full(len(self._cols), self._wshared, dtype=self.dtype)

@@ -13,6 +13,7 @@
 #include <cstring>
 #include <functional>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -96,6 +97,86 @@ template <typename F> void parallel_for(int64_t n, F f, int64_t grain = (int64_t
 static int parallel_parts(int64_t n, int64_t grain = (int64_t)1 << 22) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(std::min<unsigned>(32u, std::max(1u, std::thread::hardware_concurrency())),
                                                        (n + grain - 1) / grain));
+}
+
+// Pinned blocks that results are read back through, shared by all networks of
+// the process: at most kPinBlocks are kept while any network is alive, and the
+// last one to go frees them.  A caller owns a block between take() and give();
+// null when host memory cannot be pinned (the callers then copy directly).
+constexpr size_t kPinBytes = (size_t)1 << 20;
+constexpr size_t kPinBlocks = 8;
+struct PinPool {
+    std::mutex mu;
+    std::vector<void *> idle;
+    int64_t nets = 0;
+    void *take() {
+        {
+            std::lock_guard<std::mutex> l(mu);
+            if (!idle.empty()) { void *p = idle.back(); idle.pop_back(); return p; }
+        }
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, kPinBytes, cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        return p;
+    }
+    void give(void *p) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> l(mu);
+            if (nets > 0 && idle.size() < kPinBlocks) { idle.push_back(p); return; }
+        }
+        cudaFreeHost(p);
+    }
+    void net_born() { std::lock_guard<std::mutex> l(mu); ++nets; }
+    void net_gone() {
+        std::vector<void *> drop;
+        { std::lock_guard<std::mutex> l(mu); if (--nets == 0) drop.swap(idle); }
+        for (void *p : drop) cudaFreeHost(p);
+    }
+};
+static PinPool &pin_pool() { static PinPool *p = new PinPool(); return *p; }    // (outlives the driver's own teardown)
+struct PinBlock {
+    char *p;
+    PinBlock() : p((char *)pin_pool().take()) {}
+    ~PinBlock() { pin_pool().give(p); }
+    PinBlock(const PinBlock &) = delete;
+    PinBlock &operator=(const PinBlock &) = delete;
+};
+
+// Device memory to the host, after all work on it has finished.  Large reads go
+// through the pinned blocks by several threads, each with its own stream, so
+// that one thread's copy off the device overlaps the others' copies into the
+// destination (whose pages are often touched for the first time: 164 MB took
+// 66 ms through one pageable copy and a widening loop, and 11 ms this way in the
+// connection's own type).
+static cudaError_t read_back(int device, void *dst, const void *src, size_t bytes) {
+    const size_t chunks = (bytes + kPinBytes - 1) / kPinBytes;
+    const int nt = (int)std::min<size_t>(std::min<size_t>(kPinBlocks, std::max(1u, std::thread::hardware_concurrency())), chunks / 4);
+    if (nt <= 1) return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+    std::vector<cudaError_t> err(nt, cudaSuccess);
+    auto work = [&](int t) {
+        cudaError_t e = cudaSetDevice(device);
+        cudaStream_t st = nullptr;
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        PinBlock b;
+        for (size_t c = t; c < chunks && e == cudaSuccess; c += nt) {
+            const size_t off = c * kPinBytes, len = std::min(kPinBytes, bytes - off);
+            if (!b.p) { e = cudaMemcpy((char *)dst + off, (const char *)src + off, len, cudaMemcpyDeviceToHost); continue; }
+            e = cudaMemcpyAsync(b.p, (const char *)src + off, len, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e == cudaSuccess) std::memcpy((char *)dst + off, b.p, len);
+        }
+        if (st) cudaStreamDestroy(st);
+        err[t] = e;
+    };
+    std::vector<std::thread> th;
+    th.reserve(nt);
+    for (int t = 1; t < nt; ++t) {
+        try { th.emplace_back(work, t); } catch (...) { work(t); }      // no thread to be had: its share here
+    }
+    work(0);
+    for (auto &x : th) x.join();
+    for (cudaError_t e : err) if (e != cudaSuccess) return e;
+    return cudaSuccess;
 }
 
 // device helpers of the network set-up (grid-stride loops)
@@ -201,7 +282,7 @@ struct bg_net {
     cudaEvent_t stage_ev[2] = {nullptr, nullptr};
     bool stage_used[2] = {false, false};
     uint32_t *dMonWords = nullptr;      // persistent path with spike monitors: spike words per step of a chunk
-    long long *dMonOff = nullptr;       //   and per-step record offsets
+    long long *dMonOff = nullptr;       //   and per-step record offsets, then the counting blocks' ticket
     cudaStream_t stream = nullptr;
     std::vector<HGroup> groups; std::vector<HConn> conns; std::vector<HStdp> stdps; std::vector<HSyn> syns;
     std::vector<HSpikeMon> smons; std::vector<HStateMon> stmons; std::vector<Item> items;
@@ -958,10 +1039,7 @@ int reset_dynamic(bg_net *net) {
     return BG_OK;
 }
 
-int check_device_error(bg_net *net) {
-    DevCtl h;
-    BG_CUDA(cudaMemcpyAsync(&h, net->dCtl, sizeof(h), cudaMemcpyDeviceToHost, net->stream));
-    BG_CUDA(cudaStreamSynchronize(net->stream));
+int check_ctl(bg_net *net, const DevCtl &h) {
     if (h.err) net->failed = true;       // the network's device state is no longer consistent
     if (h.err == BG_DERR_MONITOR_OVERFLOW) return fail(BG_ESTATE, "spike monitor buffer overflow");
     if (h.err == BG_DERR_TIMEOUT) return fail(BG_ETIMEOUT, "inter-block wait timed out at step " + std::to_string(h.err_info));
@@ -971,6 +1049,13 @@ int check_device_error(bg_net *net) {
     if (h.err == BG_DERR_RANGE) return fail(BG_EINVAL, "device range check failed (entry " + std::to_string(h.err_info) + ")");
     if (h.err) return fail(BG_ESTATE, "device error " + std::to_string(h.err));
     return BG_OK;
+}
+
+int check_device_error(bg_net *net) {
+    DevCtl h;
+    BG_CUDA(cudaMemcpyAsync(&h, net->dCtl, sizeof(h), cudaMemcpyDeviceToHost, net->stream));
+    BG_CUDA(cudaStreamSynchronize(net->stream));
+    return check_ctl(net, h);
 }
 
 // NaN/inf in the first n entries of each of the nvar rows (stride npad) of a
@@ -998,6 +1083,24 @@ int check_finite_states(bg_net *n) {
 
 // Copy monitor records of the finished chunk to host memory.
 // `tail_done_upto`: last step whose 'end' slot has run.
+// `cnt` records (steps relative to base_cs) to the end of a monitor's own.
+void append_records(HSpikeMon &m, const int32_t *idx, const int32_t *steps, int64_t cnt, long long base_cs) {
+    m.idx.insert(m.idx.end(), idx, idx + cnt);
+    const size_t o = m.steps.size();
+    m.steps.resize(o + cnt);
+    for (int64_t k = 0; k < cnt; ++k) m.steps[o + k] = base_cs + steps[k];
+}
+
+// `cnt` records of a monitor's buffer from entry `first` on.
+int take_records(bg_net *net, HSpikeMon &m, int64_t first, int64_t cnt, long long base_cs) {
+    if (cnt <= 0) return BG_OK;
+    std::unique_ptr<int32_t[]> idx(new int32_t[cnt]), st(new int32_t[cnt]);
+    BG_CUDA(read_back(net->device, idx.get(), m.dIdx + first, cnt * 4));
+    BG_CUDA(read_back(net->device, st.get(), m.dSteps + first, cnt * 4));
+    append_records(m, idx.get(), st.get(), cnt, base_cs);
+    return BG_OK;
+}
+
 // Move one spike monitor's device records (steps relative to
 // chunk_base_cs) to host memory and empty its buffer.
 int drain_spikemon(bg_net *net, HSpikeMon &m, long long chunk_base_cs) {
@@ -1005,10 +1108,8 @@ int drain_spikemon(bg_net *net, HSpikeMon &m, long long chunk_base_cs) {
     BG_CUDA(cudaMemcpy(&cnt, m.dCnt, 8, cudaMemcpyDeviceToHost));
     if (cnt > m.cap) return fail(BG_ESTATE, "spike monitor buffer overflow");
     if (cnt > 0) {
-        std::vector<int32_t> idx(cnt), st(cnt);
-        BG_CUDA(cudaMemcpy(idx.data(), m.dIdx, cnt * 4, cudaMemcpyDeviceToHost));
-        BG_CUDA(cudaMemcpy(st.data(), m.dSteps, cnt * 4, cudaMemcpyDeviceToHost));
-        for (long long k = 0; k < cnt; ++k) { m.idx.push_back(idx[k]); m.steps.push_back(chunk_base_cs + st[k]); }
+        int st = take_records(net, m, 0, cnt, chunk_base_cs);
+        if (st) return st;
         long long z = 0;
         BG_CUDA(cudaMemcpy(m.dCnt, &z, 8, cudaMemcpyHostToDevice));
     }
@@ -1450,7 +1551,8 @@ int build_persist(bg_net *net) {
         a.mon_stride = g.npad / 32;
         if (!net->dMonWords &&
             (net->alloc(&net->dMonWords, (size_t)kPersistMonSteps * a.mon_stride * 4) != cudaSuccess ||
-             net->alloc(&net->dMonOff, (size_t)kPersistMonSteps * 8) != cudaSuccess))
+             net->alloc(&net->dMonOff, (size_t)(kPersistMonSteps + 1) * 8) != cudaSuccess ||
+             cudaMemsetAsync(net->dMonOff + kPersistMonSteps, 0, 8, net->stream) != cudaSuccess))
             return fail(BG_ENOMEM, "spike words");
         a.mon_words = net->dMonWords;
     }
@@ -1621,7 +1723,8 @@ int build_syn_persist(bg_net *net) {
         a.mon_stride = g.npad / 32;
         if (!net->dMonWords &&
             (net->alloc(&net->dMonWords, (size_t)kPersistMonSteps * a.mon_stride * 4) != cudaSuccess ||
-             net->alloc(&net->dMonOff, (size_t)kPersistMonSteps * 8) != cudaSuccess))
+             net->alloc(&net->dMonOff, (size_t)(kPersistMonSteps + 1) * 8) != cudaSuccess ||
+             cudaMemsetAsync(net->dMonOff + kPersistMonSteps, 0, 8, net->stream) != cudaSuccess))
             return fail(BG_ENOMEM, "spike words");
         a.mon_words = net->dMonWords;
     }
@@ -1647,13 +1750,19 @@ int build_syn_persist(bg_net *net) {
 
 // Runs nsteps with the persistent kernel (one launch) and advances the step
 // counter on the host and device.
-int run_persist(bg_net *n, int64_t nsteps) {
+int launch_persist(bg_net *n, int64_t nsteps) {
     cudaError_t e = n->persist(n->stream, (int)nsteps);
     if (e != cudaSuccess) return fail(BG_ECUDA, std::string("persistent launch: ") + cudaGetErrorString(e));
     n->launches += 1;
     n->nstep += nsteps;
     long long ns = n->nstep;
     BG_CUDA(cudaMemcpyAsync(&n->dCtl->nstep, &ns, 8, cudaMemcpyHostToDevice, n->stream));
+    return BG_OK;
+}
+
+int run_persist(bg_net *n, int64_t nsteps) {
+    int st = launch_persist(n, nsteps);
+    if (st) return st;
     BG_CUDA(cudaStreamSynchronize(n->stream));
     return BG_OK;
 }
@@ -1688,6 +1797,7 @@ int bg_net_create(int device, int precision, int deterministic, double dt, bg_ne
     if (n->alloc(&n->dCtl, sizeof(DevCtl)) != cudaSuccess) { delete n; return fail(BG_ENOMEM, "ctl"); }
     cudaMemset(n->dCtl, 0, sizeof(DevCtl));
     cudaEventCreate(&n->ev0); cudaEventCreate(&n->ev1);
+    pin_pool().net_born();
     *out = n;
     return BG_OK;
 }
@@ -1710,6 +1820,7 @@ int bg_net_destroy(bg_net *n) {
     if (n->side) cudaStreamDestroy(n->side);
     if (n->stream) cudaStreamDestroy(n->stream);
     delete n;
+    pin_pool().net_gone();
     return BG_OK;
 }
 
@@ -1993,10 +2104,24 @@ int bg_conn_get_weights(bg_net *n, int32_t cid, double *out) {
     expand_shared_weight(c);
     if (n->prepared) {
         BG_CUDA(cudaStreamSynchronize(n->stream));
-        BG_CUDA(cudaMemcpy(c.w.data(), c.dW, c.w.size(), cudaMemcpyDeviceToHost));
+        BG_CUDA(read_back(n->device, c.w.data(), c.dW, c.w.size()));
     }
-    for (int64_t k = 0; k < cnt; ++k)
-        out[k] = c.w_bits == 64 ? ((const double *)c.w.data())[k] : (double)((const float *)c.w.data())[k];
+    parallel_for(cnt, [&](int64_t lo, int64_t hi, int) {
+        if (c.w_bits == 64) std::memcpy(out + lo, c.w.data() + lo * 8, (hi - lo) * 8);
+        else for (int64_t k = lo; k < hi; ++k) out[k] = (double)((const float *)c.w.data())[k];
+    });
+    return BG_OK;
+}
+
+int bg_conn_read_weights(bg_net *n, int32_t cid, void *out, int64_t bytes) {
+    if (!n || cid < 0 || cid >= (int32_t)n->conns.size() || !out) return fail(BG_EINVAL, "bg_conn_read_weights");
+    HConn &c = n->conns[cid];
+    expand_shared_weight(c);
+    if (bytes != (int64_t)c.w.size()) return fail(BG_EINVAL, "bg_conn_read_weights: size of the connection's weights");
+    if (!n->prepared) { std::memcpy(out, c.w.data(), c.w.size()); return BG_OK; }
+    BG_CUDA(cudaSetDevice(n->device));
+    BG_CUDA(cudaStreamSynchronize(n->stream));
+    BG_CUDA(read_back(n->device, out, c.dW, c.w.size()));
     return BG_OK;
 }
 
@@ -2772,6 +2897,74 @@ int bg_net_run(bg_net *n, int64_t nsteps, int64_t cs0) {
     return st;
 }
 
+// The records of the persistent launch of c steps just enqueued, for one
+// monitor.  Usually they fit the monitor's (empty) buffer: the conversion, the
+// device's error word, the number of records and the first kRec of them (written
+// to the pinned block by a kernel, no more of them than there are) then come back
+// with one wait: 100 steps of 1000 neurons, 331 -> 238 us with the states read
+// afterwards.  Else (or without pinned memory) step ranges that fit are written
+// and read one after the other; a step alone always fits (at most m.n records,
+// cap >= m.n).
+static int persist_records(bg_net *n, HSpikeMon &m, int64_t c, long long base_cs) {
+    const HGroup &g = n->groups[0];
+    constexpr int64_t kRec = 65536;
+    constexpr size_t kCntOff = 1024, kIdxOff = 2048, kStepOff = kIdxOff + kRec * 4;
+    static_assert(sizeof(DevCtl) <= kCntOff && kStepOff + kRec * 4 <= kPinBytes, "read-back block");
+    bg::MonWordsArgs w;
+    w.ctl = n->dCtl; w.words = n->dMonWords; w.stride = g.npad / 32; w.nsteps = (int)c; w.s0 = 0;
+    w.origin = m.origin; w.n = m.n; w.cnt = m.dCnt; w.cap = m.cap; w.idx = m.dIdx; w.steps = m.dSteps;
+    w.off = n->dMonOff; w.ticket = (unsigned int *)(n->dMonOff + kPersistMonSteps);
+    w.base0 = 0; w.whole = 1;
+    bg::k_monw_count<<<(unsigned)c, bg::kMonWordsThreads, 0, n->stream>>>(w);
+    BG_CUDA(cudaGetLastError());
+    n->launches += 1;
+    PinBlock pin;
+    long long tot = -1;
+    if (pin.p) {
+        const int64_t rec = std::min(m.cap, kRec);
+        bg::k_monw_write<<<(unsigned)c, bg::kMonWordsThreads, 0, n->stream>>>(w);    // (nothing when the records do not fit)
+        bg::k_monw_pack<<<16, 256, 0, n->stream>>>(w, (DevCtl *)pin.p, (long long *)(pin.p + kCntOff), (int32_t *)(pin.p + kIdxOff),
+                                                   (int32_t *)(pin.p + kStepOff), rec);
+        BG_CUDA(cudaGetLastError());
+        n->launches += 2;
+        BG_CUDA(cudaMemsetAsync(m.dCnt, 0, 8, n->stream));
+        BG_CUDA(cudaStreamSynchronize(n->stream));
+        DevCtl h;
+        std::memcpy(&h, pin.p, sizeof(h));
+        int st = check_ctl(n, h);
+        if (st) return st;
+        std::memcpy(&tot, pin.p + kCntOff, 8);
+        if (tot <= m.cap) {
+            const int64_t first = std::min<int64_t>(tot, rec);
+            append_records(m, (const int32_t *)(pin.p + kIdxOff), (const int32_t *)(pin.p + kStepOff), first, base_cs);
+            return tot > first ? take_records(n, m, first, tot - first, base_cs) : BG_OK;
+        }
+    } else {
+        BG_CUDA(cudaMemcpyAsync(&tot, m.dCnt, 8, cudaMemcpyDeviceToHost, n->stream));
+        BG_CUDA(cudaMemsetAsync(m.dCnt, 0, 8, n->stream));
+    }
+    std::vector<long long> off(c + 1);
+    BG_CUDA(cudaMemcpyAsync(off.data(), n->dMonOff, c * 8, cudaMemcpyDeviceToHost, n->stream));
+    BG_CUDA(cudaStreamSynchronize(n->stream));
+    off[c] = tot;
+    w.whole = 0;
+    for (int64_t s0 = 0; s0 < c;) {
+        int64_t s1 = s0;
+        while (s1 < c && off[s1 + 1] - off[s0] <= m.cap) ++s1;
+        bg::MonWordsArgs r = w;
+        r.words = n->dMonWords + s0 * w.stride; r.off = n->dMonOff + s0; r.base0 = off[s0];
+        r.nsteps = (int)(s1 - s0); r.s0 = (int)s0;
+        bg::k_monw_write<<<(unsigned)(s1 - s0), bg::kMonWordsThreads, 0, n->stream>>>(r);
+        BG_CUDA(cudaGetLastError());
+        n->launches += 1;
+        int st = check_device_error(n);  // (waits)
+        if (!st) st = take_records(n, m, 0, off[s1] - off[s0], base_cs);
+        if (st) return st;
+        s0 = s1;
+    }
+    return BG_OK;
+}
+
 static int net_run_steps(bg_net *n, int64_t nsteps, int64_t cs0) {
     if (!n->prepared) { int st = bg_net_prepare(n); if (st) return st; }
     if (nsteps == 0) return BG_OK;
@@ -2786,44 +2979,13 @@ static int net_run_steps(bg_net *n, int64_t nsteps, int64_t cs0) {
         const bool mons = !n->smons.empty();
         int64_t chunk = mons ? kPersistMonSteps : (int64_t)1 << 20;
         if (!n->stmons.empty()) chunk = std::min<int64_t>(chunk, n->chunk_steps);   // rows of the monitor buffers
-        std::vector<long long> cnt;
         for (int64_t done = 0; done < nsteps;) {
             const int64_t c = std::min(chunk, nsteps - done);
-            int st = run_persist(n, c);
+            int st = mons ? launch_persist(n, c) : run_persist(n, c);
             if (st) return st;
-            if (mons) {
-                const HGroup &g = n->groups[0];
-                for (auto &m : n->smons) {
-                    bg::MonWordsArgs w;
-                    w.ctl = n->dCtl; w.words = n->dMonWords; w.stride = g.npad / 32; w.nsteps = (int)c; w.s0 = 0;
-                    w.origin = m.origin; w.n = m.n; w.cnt = m.dCnt; w.cap = m.cap; w.idx = m.dIdx; w.steps = m.dSteps;
-                    w.off = n->dMonOff;
-                    bg::k_monw_count<<<(unsigned)c, bg::kMonWordsThreads, 0, n->stream>>>(w);
-                    BG_CUDA(cudaGetLastError());
-                    n->launches += 1;
-                    cnt.resize(c);
-                    BG_CUDA(cudaMemcpyAsync(cnt.data(), n->dMonOff, c * 8, cudaMemcpyDeviceToHost, n->stream));
-                    BG_CUDA(cudaStreamSynchronize(n->stream));
-                    // step ranges whose records fit the (empty) buffer; a step
-                    // alone always fits (at most m.n records, cap >= m.n)
-                    for (int64_t s0 = 0; s0 < c;) {
-                        int64_t s1 = s0, tot = 0;
-                        while (s1 < c && tot + cnt[s1] <= m.cap) tot += cnt[s1++];
-                        bg::MonWordsArgs r = w;
-                        r.words = n->dMonWords + s0 * w.stride; r.off = n->dMonOff + s0;
-                        r.nsteps = (int)(s1 - s0); r.s0 = (int)s0;
-                        bg::k_monw_scan<<<1, bg::kMonWordsThreads, 0, n->stream>>>(r);
-                        bg::k_monw_write<<<(unsigned)(s1 - s0), bg::kMonWordsThreads, 0, n->stream>>>(r);
-                        BG_CUDA(cudaGetLastError());
-                        n->launches += 2;
-                        BG_CUDA(cudaStreamSynchronize(n->stream));
-                        st = check_device_error(n);
-                        if (st) return st;
-                        st = drain_spikemon(n, m, cs0 + done);
-                        if (st) return st;
-                        s0 = s1;
-                    }
-                }
+            for (auto &m : n->smons) {
+                st = persist_records(n, m, c, cs0 + done);
+                if (st) return st;
             }
             // the launch ran the 'end' slot of its last step
             if (!n->stmons.empty()) { st = drain(n, cs0 + done, n->nstep - 1, off0); if (st) return st; }
@@ -2892,8 +3054,21 @@ int bg_group_get_state(bg_net *n, int32_t gid, int var, double *out) {
     if (!gid_ok(n, gid) || var < 0 || var >= n->groups[gid].nvar || !out) return fail(BG_EINVAL, "bg_group_get_state");
     HGroup &g = n->groups[gid];
     if (!n->prepared) { std::memcpy(out, g.S0.data() + (size_t)var * g.n, g.n * 8); return BG_OK; }
+    const size_t ts = tsize(n), bytes = (size_t)g.n * ts;
+    const char *src = (const char *)g.dS + (size_t)var * g.npad * ts;
+    if (bytes <= kPinBytes) {
+        // in order on the network's own stream, one wait
+        PinBlock pin;
+        if (pin.p) {
+            BG_CUDA(cudaMemcpyAsync(pin.p, src, bytes, cudaMemcpyDeviceToHost, n->stream));
+            BG_CUDA(cudaStreamSynchronize(n->stream));
+            if (ts == 8) std::memcpy(out, pin.p, bytes);
+            else for (int64_t i = 0; i < g.n; ++i) out[i] = ((const float *)pin.p)[i];
+            return BG_OK;
+        }
+    }
     BG_CUDA(cudaStreamSynchronize(n->stream));
-    if (n->precision == 64) BG_CUDA(cudaMemcpy(out, (double *)g.dS + (size_t)var * g.npad, g.n * 8, cudaMemcpyDeviceToHost));
+    if (n->precision == 64) BG_CUDA(cudaMemcpy(out, src, bytes, cudaMemcpyDeviceToHost));
     else {
         std::vector<float> tmp(g.n);
         BG_CUDA(cudaMemcpy(tmp.data(), (float *)g.dS + (size_t)var * g.npad, g.n * 4, cudaMemcpyDeviceToHost));
@@ -3474,23 +3649,32 @@ int batch_collect(bg_batch *b, const std::vector<int32_t> &out, const std::vecto
         BG_CUDA(cudaMemcpyAsync(b->dGather, g.data(), g.size() * 8, cudaMemcpyHostToDevice, b->stream));
         k_batch_gather<<<(unsigned)std::min(nreg, 4096), 256, 0, b->stream>>>(src, b->dGather, nreg, dst);
         BG_CUDA(cudaGetLastError());
-        BG_CUDA(cudaStreamSynchronize(b->stream));
         return BG_OK;
     };
     if (tot > 0) {
         int st = gather((const uint32_t *)b->dSIdx, (uint32_t *)b->dCIdx, so, len, dof, 1); if (st) return st;
         st = gather((const uint32_t *)b->dSStep, (uint32_t *)b->dCStep, so, len, dof, 1); if (st) return st;
-        std::vector<int32_t> idx(tot), stp(tot);
-        BG_CUDA(cudaMemcpy(idx.data(), b->dCIdx, tot * 4, cudaMemcpyDeviceToHost));
-        BG_CUDA(cudaMemcpy(stp.data(), b->dCStep, tot * 4, cudaMemcpyDeviceToHost));
-        int64_t p = 0;
-        for (size_t i = 0; i < nn; ++i)
-            for (int m = 0; m < (int)b->nets[i]->smons.size(); ++m) {
-                HSpikeMon &h = b->nets[i]->smons[m];
-                const int64_t c = out[i * K + 1 + m];
-                const long long cs = t0[i] + off[i];
-                for (int64_t k = 0; k < c; ++k, ++p) { h.idx.push_back(idx[p]); h.steps.push_back(cs + stp[p]); }
+        BG_CUDA(cudaStreamSynchronize(b->stream));
+        std::unique_ptr<int32_t[]> idx(new int32_t[tot]), stp(new int32_t[tot]);
+        BG_CUDA(read_back(b->device, idx.get(), b->dCIdx, tot * 4));
+        BG_CUDA(read_back(b->device, stp.get(), b->dCStep, tot * 4));
+        std::vector<int64_t> pos(nn + 1, 0);
+        for (size_t i = 0; i < nn; ++i) {
+            pos[i + 1] = pos[i];
+            for (int m = 0; m < (int)b->nets[i]->smons.size(); ++m) pos[i + 1] += out[i * K + 1 + m];
+        }
+        // (each network's records are its own: threads over the networks, about 2^18 records each)
+        const int64_t grain = std::max<int64_t>(1, (int64_t)(((int64_t)1 << 18) * (int64_t)nn / tot));
+        parallel_for((int64_t)nn, [&](int64_t lo, int64_t hi, int) {
+            for (int64_t i = lo; i < hi; ++i) {
+                int64_t p = pos[i];
+                for (int m = 0; m < (int)b->nets[i]->smons.size(); ++m) {
+                    const int64_t c = out[i * K + 1 + m];
+                    append_records(b->nets[i]->smons[m], idx.get() + p, stp.get() + p, c, t0[i] + off[i]);
+                    p += c;
+                }
             }
+        }, grain);
     }
     // state rows
     so.clear(); len.clear(); dof.clear(); tot = 0;
@@ -3503,6 +3687,7 @@ int batch_collect(bg_batch *b, const std::vector<int32_t> &out, const std::vecto
     if (tot > 0) {
         const int words = (int)(sizeof(T) / 4);
         int st = gather((const uint32_t *)b->dRows, (uint32_t *)b->dCRows, so, len, dof, words); if (st) return st;
+        BG_CUDA(cudaStreamSynchronize(b->stream));
         BG_CUDA(cudaMemcpy(vals.data(), b->dCRows, tot * sizeof(T), cudaMemcpyDeviceToHost));
     }
     int64_t p = 0;

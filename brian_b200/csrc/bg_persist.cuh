@@ -391,8 +391,9 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
 // ---- spike monitors of the persistent path ---------------------------------
 // After a launch of nsteps steps, the words it wrote become the monitor's
 // (step, index) records in the order of k_spikemon (steps ascending, indices
-// ascending within a step): per-step counts, one scan over the steps, then
-// one block per step writes its records at its offset.
+// ascending within a step): per-step counts, one scan over the steps (by the
+// block that counted last), then one block per step writes its records at its
+// offset.
 struct MonWordsArgs {
     DevCtl *ctl;
     const uint32_t *words; int64_t stride; int nsteps;
@@ -400,11 +401,15 @@ struct MonWordsArgs {
     int64_t origin, n;                    // monitored range of the group
     long long *cnt; int64_t cap; int32_t *idx; int32_t *steps;
     long long *off;                       // [nsteps] per-step record offsets (scratch)
+    unsigned int *ticket;                 // blocks that have counted (0 between launches)
+    long long base0; int whole;           // offset of words[0]'s first record; all steps of the launch in one go
 };
 constexpr int kMonWordsThreads = 1024;
 
 __global__ void __launch_bounds__(kMonWordsThreads) k_monw_count(const MonWordsArgs a) {
     __shared__ int wsum[kMonWordsThreads / 32];
+    __shared__ long long wbase[kMonWordsThreads / 32];
+    __shared__ bool last;
     const int s = blockIdx.x, tid = threadIdx.x;
     const uint32_t *H = a.words + (int64_t)s * a.stride;
     const int64_t end = a.origin + a.n, w0 = a.origin >> 5, w1 = (end + 31) >> 5;
@@ -418,37 +423,40 @@ __global__ void __launch_bounds__(kMonWordsThreads) k_monw_count(const MonWordsA
         int v = wsum[tid];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (tid == 0) a.off[s] = v;
+        if (tid == 0) {
+            a.off[s] = v;
+            __threadfence();
+            last = atomicAdd(a.ticket, 1u) + 1u == gridDim.x;
+        }
     }
-}
-
-// one block: exclusive scan of the per-step counts from the buffer's fill
-// level; advances the fill level (nsteps <= kMonWordsThreads)
-__global__ void __launch_bounds__(kMonWordsThreads) k_monw_scan(const MonWordsArgs a) {
-    __shared__ long long wsum[kMonWordsThreads / 32 + 1];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const long long v = tid < a.nsteps ? a.off[tid] : 0;
+    __syncthreads();
+    if (!last) return;
+    // exclusive scan of the counts (nsteps <= kMonWordsThreads); the total to cnt
+    __threadfence();
+    const int lane = tid & 31;
+    const long long v = tid < a.nsteps ? *(volatile long long *)(a.off + tid) : 0;
     long long incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) { const long long x = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += x; }
-    if (lane == 31) wsum[tid >> 5] = incl;
+    if (lane == 31) wbase[tid >> 5] = incl;
     __syncthreads();
     if (tid == 0) {
-        long long r = *a.cnt;
-        for (int q = 0; q < kMonWordsThreads / 32; ++q) { const long long x = wsum[q]; wsum[q] = r; r += x; }
-        wsum[kMonWordsThreads / 32] = r;
+        long long r = 0;
+        for (int q = 0; q < kMonWordsThreads / 32; ++q) { const long long x = wbase[q]; wbase[q] = r; r += x; }
+        *a.cnt = r;
+        *a.ticket = 0;
     }
     __syncthreads();
-    if (tid < a.nsteps) a.off[tid] = wsum[tid >> 5] + incl - v;
-    if (tid == 0) *a.cnt = wsum[kMonWordsThreads / 32];
+    if (tid < a.nsteps) a.off[tid] = wbase[tid >> 5] + incl - v;
 }
 
 __global__ void __launch_bounds__(kMonWordsThreads) k_monw_write(const MonWordsArgs a) {
     __shared__ int wcnt[kMonWordsThreads / 32 + 1];
+    if (a.whole && *a.cnt > a.cap) return;       // the host takes smaller ranges of steps
     const int s = blockIdx.x, tid = threadIdx.x;
     const uint32_t *H = a.words + (int64_t)s * a.stride;
     const int64_t end = a.origin + a.n, w0 = a.origin >> 5, w1 = (end + 31) >> 5;
-    long long base = a.off[s];
+    long long base = a.off[s] - a.base0;
     for (int64_t cw = w0; cw < w1; cw += kMonWordsThreads) {
         const int64_t wi = cw + tid;
         uint32_t word = wi < w1 ? masked_word(H, wi, a.origin, end) : 0u;
@@ -470,6 +478,17 @@ __global__ void __launch_bounds__(kMonWordsThreads) k_monw_write(const MonWordsA
         base += wcnt[kMonWordsThreads / 32];
         __syncthreads();
     }
+}
+
+// The error word, the number of records and the first `rec` of them into a
+// pinned block of the host (five small copies' latencies otherwise).
+__global__ void __launch_bounds__(256) k_monw_pack(const MonWordsArgs a, DevCtl *ctl, long long *cnt, int32_t *idx, int32_t *steps,
+                                                  int64_t rec) {
+    const long long tot = *a.cnt;
+    const int64_t n = tot > a.cap ? 0 : (tot < rec ? tot : rec);
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t == 0) { *ctl = *a.ctl; *cnt = tot; }
+    for (int64_t i = t; i < n; i += (int64_t)gridDim.x * blockDim.x) { idx[i] = a.idx[i]; steps[i] = a.steps[i]; }
 }
 
 }  // namespace bg

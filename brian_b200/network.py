@@ -110,7 +110,7 @@ class _Binding(object):
         self.rt.set_state(self.gids[grp], var, values)
 
     def read_weights(self, c):
-        return self.rt.conn_get_weights(self.cids[c], c._nnz())
+        return self.rt.conn_read_weights(self.cids[c], c._nnz(), c.dtype)
 
     def write_weights(self, c, w):
         self.rt.conn_set_weights(self.cids[c], w)

@@ -168,6 +168,8 @@ BG_API int bg_conn_add_dense(bg_net *net, int32_t src_gid, int64_t src_origin,
 /* Weights in the connection's own order (CSR data order, or row-major for
  * dense), widened to double. */
 BG_API int bg_conn_get_weights(bg_net *net, int32_t cid, double *out);
+/* The same weights in the connection's own type; bytes: their whole size. */
+BG_API int bg_conn_read_weights(bg_net *net, int32_t cid, void *out, int64_t bytes);
 BG_API int bg_conn_set_weights(bg_net *net, int32_t cid, const double *in);
 
 /* ExponentialSTDP / STDP (stdp.py:181-539) on a non-delayed connection.
