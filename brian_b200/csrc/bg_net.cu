@@ -244,7 +244,7 @@ struct HSyn {
     int32_t *dDoff = nullptr;           // per source, start of each delay in its row (when it fits 256 MB)
     int nbins = 0;
     int32_t *dSlist = nullptr; int *dScnt = nullptr; int sdepth = 0;   // spike lists of the last sdepth steps
-    double *dTermSrc = nullptr;         // persistent kernel: the statement's term per synapse, by-source order
+    bg::SynRec *dRec = nullptr;         // persistent kernel: target, delay and term per synapse, by source
     // synapses with code (bg_synapses_set_code): synaptic variables [nsv][nsyn]
     // (synapse order on the host, column order on the device), the generated
     // pre/post code, the target variables it uses (slots; `writes` those it
@@ -314,8 +314,11 @@ struct bg_net {
         size_t smem = 0;
     } cluster;
     unsigned int *dArrived = nullptr;
-    int *dUsePull3 = nullptr;           // Synapses persistent kernel: overflow flags by step mod 3
-    int *dPBinCnt = nullptr; unsigned long long *dPBinKey = nullptr; double *dPBinT = nullptr;   //   and its bins
+    // Synapses persistent kernel: the ring of bins, to be filled again from
+    // the history before the next launch when stale
+    int *dRingCnt = nullptr; bg::SynRec *dRingEv = nullptr; size_t ring_bins = 0;
+    bool syn_ring_stale = true;
+    std::function<int()> refill_ring;
     int64_t launches = 0; double last_ms = 0;
     unsigned int spin_limit = BG_SPIN_LIMIT;   // polls of a bounded inter-block wait
     int hold_block = -1;                // test hook: a persistent block that never arrives
@@ -1007,7 +1010,7 @@ int reset_lazy(bg_net *net) {
 }
 
 int reset_dynamic(bg_net *net) {
-    net->syn_lists_stale = true;
+    net->syn_lists_stale = net->syn_ring_stale = true;
     int lst = reset_lazy(net);
     if (lst) return lst;
     for (auto &g : net->groups) {
@@ -1581,12 +1584,14 @@ int build_persist(bg_net *net) {
     return BG_OK;
 }
 
-// The persistent kernel's copy of a Synapses object's terms in by-source
-// order (its one statement), from the column-order terms on the device.
-int refresh_term_src(bg_net *net, const HSyn &y) {
-    if (!y.dTermSrc || y.nsyn == 0) return BG_OK;
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((y.nsyn + 255) / 256, (int64_t)sm_count() * 8));
-    bg::k_syn_term_src<<<grid, 256, 0, net->stream>>>(y.dSq, y.dTerm, y.nsyn, y.dTermSrc);
+// The persistent kernel's records of a Synapses object, with its one
+// statement's terms as they are on the device.
+int refresh_records(bg_net *net, int yi) {
+    const HSyn &y = net->syns[yi];
+    net->syn_ring_stale = true;              // (events on their way carry the terms)
+    if (!y.dRec || y.nsyn == 0) return BG_OK;
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((y.sn + 7) / 8, (int64_t)sm_count() * 8));
+    bg::k_synp_records<<<grid, 256, 0, net->stream>>>(syn_ev_args(net, yi), yi, y.dRec);
     BG_CUDA(cudaGetLastError());
     BG_CUDA(cudaStreamSynchronize(net->stream));
     return BG_OK;
@@ -1625,6 +1630,10 @@ int build_syn_persist(bg_net *net) {
     if (!syn_persist_shape(net)) return BG_OK;
     for (const HSyn &y : net->syns)
         if (!y.events || !y.dScnt) return BG_OK;
+    // a record holds a synapse's place in its source's row in 20 bits
+    for (const HSyn &y : net->syns)
+        for (int64_t i = 0; i < y.sn; ++i)
+            if (y.srcptr[i + 1] - y.srcptr[i] > ((int64_t)1 << 20)) return BG_OK;
     const HGroup &g = net->groups[0];
     {
         int dev = 0, coop = 0;
@@ -1633,7 +1642,7 @@ int build_syn_persist(bg_net *net) {
         if (!coop) return BG_OK;
     }
     const int64_t blocks = (g.n + bg::kSPBn - 1) / bg::kSPBn;
-    const size_t smem = (size_t)bg::kSynBinCap * (8 + 8);
+    const size_t smem = (size_t)bg::kSynBinCap * sizeof(bg::SynRec) + net->syns.size() * (bg::kSPBn + 1) * 4;
     const void *kern[4][2] = {{(const void *)bg::k_syn_persist<1, false>, (const void *)bg::k_syn_persist<1, true>},
                               {(const void *)bg::k_syn_persist<2, false>, (const void *)bg::k_syn_persist<2, true>},
                               {(const void *)bg::k_syn_persist<3, false>, (const void *)bg::k_syn_persist<3, true>},
@@ -1652,10 +1661,6 @@ int build_syn_persist(bg_net *net) {
     }
     if (blocks > slots) return BG_OK;
     if (!net->dArrived && net->alloc(&net->dArrived, 64) != cudaSuccess) return fail(BG_ENOMEM, "arrival counter");
-    if (!net->dUsePull3) {
-        if (net->alloc(&net->dUsePull3, 16) != cudaSuccess) return fail(BG_ENOMEM, "overflow flags");
-        BG_CUDA(cudaMemsetAsync(net->dUsePull3, 0, 16, net->stream));
-    }
     bg::SynPersistArgs a;
     std::memset(&a, 0, sizeof(a));
     a.ctl = net->dCtl; a.S = (double *)g.dS; a.n = g.n; a.npad = g.npad;
@@ -1673,31 +1678,32 @@ int build_syn_persist(bg_net *net) {
     a.nobj = (int)net->syns.size();
     const HSyn &y0 = net->syns[0];
     a.nbins = y0.nbins; a.blk0 = (int)(y0.to / bg::kSynBin); a.tn = y0.tn;
-    if (!net->dPBinCnt) {
-        if (net->alloc(&net->dPBinCnt, (size_t)2 * a.nbins * 4) != cudaSuccess ||
-            net->alloc(&net->dPBinKey, (size_t)2 * a.nbins * bg::kSynBinCap * 8) != cudaSuccess ||
-            net->alloc(&net->dPBinT, (size_t)2 * a.nbins * bg::kSynBinCap * 8) != cudaSuccess)
+    int dmax = 0;
+    for (const HSyn &y : net->syns) dmax = std::max(dmax, y.dmax);
+    a.ring = dmax + 2;
+    // entries a bin holds: all that are ordered in shared memory, or the power of two below that fits kSPRing
+    a.cap = bg::kSynBinCap;
+    while (a.cap > bg::kSPBn && (int64_t)a.ring * a.nbins * a.cap * (int64_t)sizeof(bg::SynRec) > bg::kSPRing) a.cap /= 2;
+    if (!net->dRingCnt) {
+        net->ring_bins = (size_t)a.ring * a.nbins;
+        if (net->alloc(&net->dRingCnt, net->ring_bins * 4) != cudaSuccess ||
+            net->alloc(&net->dRingEv, net->ring_bins * a.cap * sizeof(bg::SynRec)) != cudaSuccess)
             return fail(BG_ENOMEM, "synapse event bins");
-        BG_CUDA(cudaMemsetAsync(net->dPBinCnt, 0, (size_t)2 * a.nbins * 4, net->stream));
     }
-    a.bin_cnt = net->dPBinCnt; a.bin_key = net->dPBinKey; a.bin_t = net->dPBinT;
+    a.bin_cnt = net->dRingCnt; a.bin_ev = net->dRingEv;
     for (int k = 0; k < a.nobj; ++k) {
         HSyn &y = net->syns[k];
-        if (!y.dTermSrc) {
-            if (net->alloc(&y.dTermSrc, (size_t)std::max<int64_t>(1, y.nsyn) * 8) != cudaSuccess)
-                return fail(BG_ENOMEM, "synapse terms by source");
-            int st = refresh_term_src(net, y);
+        if (!y.dRec) {
+            if (net->alloc(&y.dRec, (size_t)std::max<int64_t>(1, y.nsyn) * sizeof(bg::SynRec)) != cudaSuccess)
+                return fail(BG_ENOMEM, "synapse records by source");
+            int st = refresh_records(net, k);
             if (st) return st;
         }
         bg::SynPersistObj &o = a.o[k];
         o.e = syn_ev_args(net, k);
-        o.term_src = y.dTermSrc;
+        o.rec = y.dRec;
         o.var = y.op_var[0]; o.sub = y.op_sub[0];
-        a.pair0[k + 1] = a.pair0[k] + y.dmax;
     }
-    const int npair = a.pair0[a.nobj];
-    a.nparts = npair ? std::max<int>(1, (int)(blocks / npair)) : 1;
-    a.use_pull = net->dUsePull3;
     a.spikes = net->dCounters;
     a.arrived = net->dArrived;
     a.spin_limit = net->spin_limit;
@@ -1734,12 +1740,23 @@ int build_syn_persist(bg_net *net) {
             if ((((a.anz >> (j * g.nvar + k)) & 1ull) != 0) != (j == 0 || j == k)) diag = false;
     const void *k = kern[g.nvar - 1][diag ? 1 : 0];
     unsigned int *arr = net->dArrived;
-    int *flags = net->dUsePull3;
     net->persist_used = bg::kSPTh;
-    net->persist = [a, blocks, k, smem, arr, flags](cudaStream_t s, int nsteps) {
+    net->refill_ring = [a, net]() -> int {
+        BG_CUDA(cudaMemsetAsync(net->dRingCnt, 0, net->ring_bins * 4, net->stream));
+        for (int k = 0; k < a.nobj && net->nstep > 0; ++k) {
+            const bg::SynEvArgs &e = a.o[k].e;
+            if (e.dmax == 0) continue;
+            const int64_t nw = ((e.so + e.sn + 31) / 32 - e.so / 32) * e.dmax;
+            const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((nw + 7) / 8, (int64_t)sm_count() * 8));
+            bg::k_synp_refill<<<grid, 256, 0, net->stream>>>(a, k);
+            BG_CUDA(cudaGetLastError());
+            net->launches += 1;
+        }
+        net->syn_ring_stale = false;
+        return BG_OK;
+    };
+    net->persist = [a, blocks, k, smem, arr](cudaStream_t s, int nsteps) {
         cudaError_t e = cudaMemsetAsync(arr, 0, 64, s);
-        if (e != cudaSuccess) return e;
-        e = cudaMemsetAsync(flags, 0, 16, s);
         if (e != cudaSuccess) return e;
         bg::SynPersistArgs b = a; b.nsteps = nsteps;
         void *args[] = {(void *)&b};
@@ -2305,7 +2322,7 @@ static int bg_synapses_set_terms_impl(bg_net *n, int yi, const double *terms) {
         for (int64_t p = 0; p < y.nsyn; ++p) col[(size_t)k * y.nsyn + p] = y.terms[(size_t)k * y.nsyn + y.perm[p]];
     BG_CUDA(cudaStreamSynchronize(n->stream));
     BG_CUDA(cudaMemcpy(y.dTerm, col.data(), col.size() * 8, cudaMemcpyHostToDevice));
-    return refresh_term_src(n, y);
+    return refresh_records(n, yi);
 }
 
 int bg_synapses_set_terms(bg_net *n, int32_t sid, const double *terms) {
@@ -2798,6 +2815,7 @@ static int prepare_impl(bg_net *n) {
 // The event path's spike lists of the last dmax steps, rebuilt from the
 // spike history when it did not come from the gather launches.
 static int refresh_syn_lists(bg_net *n) {
+    if (n->persist && n->refill_ring) return n->syn_ring_stale ? n->refill_ring() : BG_OK;
     if (!n->syn_lists_stale) return BG_OK;
     for (size_t yi = 0; yi < n->syns.size(); ++yi) {
         const HSyn &y = n->syns[yi];
@@ -3248,7 +3266,7 @@ int bg_net_load_state(bg_net *n, const void *buf, int64_t bytes) {
     if (!ok) { n->failed = true; return fail(BG_EINVAL, r.err + "; the network must be rebuilt"); }
     if (r.left) { n->failed = true; return fail(BG_EINVAL, "state has trailing bytes; the network must be rebuilt"); }
     n->nstep = nstep;
-    n->syn_lists_stale = true;
+    n->syn_lists_stale = n->syn_ring_stale = true;
     { int lst = reset_lazy(n); if (lst) return lst; }
     long long ns = nstep;
     BG_CUDA(cudaMemcpy(&n->dCtl->nstep, &ns, 8, cudaMemcpyHostToDevice));

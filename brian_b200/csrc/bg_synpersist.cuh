@@ -5,28 +5,34 @@
 //
 // Block b owns neurons [1024 b, 1024 b + 1024) for the whole launch, state in
 // registers (512 threads, neurons tid and tid + 512), and bin b: the events
-// of every object that reach those neurons.  A step t is
+// of every object that reach those neurons, in a ring of dmax + 2 slots by the
+// step that applies them.  A step t is
 //   A: update + threshold; the block's spike words into the history (and the
-//      monitor words); the last 32 x nobj threads append the block's spikes
-//      to each object's spike list of step t and push their delay-0 events,
-//      while the other threads push the events of the spike lists of steps
-//      t-1 .. t-dmax ((object, delay) lists dealt out over the blocks) into
-//      the bins of parity t: a key in the pull's order -- target, object,
-//      delay descending, source, rank -- and the statement's term, read in
-//      by-source order beside the target;
+//      monitor words); kSPParts warps per spike and object take all the source's
+//      synapses, whatever their delay, and put each event -- a key in the
+//      pull's order (target, object, delay descending, source, rank) and the
+//      statement's term, read as one 16-byte record by source -- into the bin
+//      of its target in slot t + d;
 //   arrive at step t (release), wait for every block's arrival (acquire);
-//   C: bin b of parity t ordered (counting sort by target, insertion sort of
-//      each target's few events by key) and applied to the registers in that
-//      order -- the additions of the pull, in its order -- the bin emptied;
-//      the resets of step t; StateMonitors ('end').
-// One wait per step: a block in A(t+1) has passed the wait of step t, so
-// every block has finished C(t-1) (the bins of parity t+1 it pushes into are
-// empty) and A(t) (the lists of step t are complete).  The overflow flags
-// form a ring of three (set in A(t), read in C(t), cleared by block 0 in
-// A(t+2)); the spike-list count of step t+1 is cleared by block 0 in A(t).
-// A step whose events overflow a bin is delivered by the pull's test for
-// every target, object by object.  Every wait is bounded; on timeout the
-// block raises BG_DERR_TIMEOUT and leaves the loop.
+//   C: bin b of slot t applied to the registers in key order -- the additions
+//      of the pull, in its order -- and emptied; the resets of step t;
+//      StateMonitors ('end').
+// One wait per step: a block in A(t+2) has passed the wait of step t+1, so every
+// block has finished C(t), where it empties its bin of slot t, which A(t+2) may
+// push into again.  A bin that more events reached than it holds is delivered by
+// the pull's test for its targets, object by object.  The ring outlives a launch; after a
+// reinit, a loaded state or changed terms it is filled again from the spike
+// history (k_synp_refill).  Every wait is bounded; on timeout the block raises
+// BG_DERR_TIMEOUT and leaves the loop.
+//
+// What bounds it: the chain of a step's dependent round trips (record, bin
+// slot, store, arrival, count and entries).  Pushing a spike's events for all
+// delays at once reads its row once and coalesced, by the block that found it;
+// walking the spike lists of every past step and each delay's part of the rows
+// again, dealt over the blocks, took two more round trips (list entry, delay
+// offsets) and gathered records one by one: 12.3 -> 5.4 us a step at 32768
+// neurons of in-degree 160.  Ordering a target's few events where they arrive
+// (kSPTab each) leaves the counting sort to the busy bins.
 #pragma once
 #include "bg_persist.cuh"
 
@@ -36,11 +42,18 @@ constexpr int kSPTh = kSynBinThreads;            // threads per block
 constexpr int kSPNpt = kSynTPT;                  // neurons per thread
 constexpr int kSPBn = kSPTh * kSPNpt;            // neurons per block
 static_assert(kSPBn == kSynBin, "a block's neurons are one bin of targets");
-constexpr int kSynSub = 4;                       // threads per listed source on the spike lists
+constexpr int kSPTab = kSynBinCap / kSPBn;       // events of one target ordered without a sort
+constexpr int kSPParts = 4;                      // warps per source: a few records a lane, loaded at once
+constexpr int64_t kSPRing = (int64_t)2 << 30;    // bytes of the ring of bins; kSynBinCap entries a bin if that fits
+
+// One synapse, rows by source.  x: target within its bin (10 bits), object (2),
+// 255 - delay (8), the target's bin (24; the source takes its place in an
+// event's key), place in the source's row (20).  y: the statement's term.
+using SynRec = ulonglong2;
 
 struct SynPersistObj {
-    SynEvArgs e;                                 // lists, rows by source, pull columns, terms
-    const double *term_src;                      // the statement's term per synapse, by-source order
+    SynEvArgs e;                                 // rows by source, pull columns, terms
+    const SynRec *rec;                           // [nsyn] by source
     int var, sub;                                // the statement: var += term (sub: var -= term)
 };
 
@@ -53,11 +66,9 @@ struct SynPersistArgs {
     int reset_kind, reset_var, reset_var2; double reset_val;
     uint32_t *hist; int depth; int64_t nwords;
     int nobj; SynPersistObj o[kSynEvMerge];
-    int pair0[kSynEvMerge + 1]; int nparts;      // (object, delay >= 1) lists dealt out: block / nparts
-    // the objects' common bins by step parity: [2][nbins], [2][nbins][cap]
-    int *bin_cnt; unsigned long long *bin_key; double *bin_t;
+    // the objects' common bins: [ring][nbins], [ring][nbins][cap]
+    int *bin_cnt; SynRec *bin_ev; int ring, cap;
     int nbins, blk0; int64_t tn;                 // bin 0 is block blk0's; targets of the range
-    int *use_pull;                               // [3] overflow flags by step mod 3
     unsigned long long *spikes;
     unsigned int *arrived;                       // [4] arrivals per step mod 4 (zeroed before the launch)
     int nsteps;
@@ -67,35 +78,73 @@ struct SynPersistArgs {
     int nrec; RecDev rec[kMaxRec];               // StateMonitors; blk_lo holds this kernel's block ranges
 };
 
-// the events of source i's synapses of delay d of object k into the bins of
-// one parity (key and term): this thread's share, synapses sub, sub + nsub,
-// ... of the source's row of that delay, four at a time (loads, then slots,
-// then stores)
-__device__ __forceinline__ void synp_push(const SynPersistObj &ob, int k, int64_t i, int d, int sub, int nsub,
-                                          int *flag, int *cnt, unsigned long long *key, double *tv) {
-    const SynEvArgs &a = ob.e;
-    int64_t r0, r1;
-    syn_src_range(a, i, d, r0, r1);
-    if (r1 - r0 > 256) { if (sub == 0) atomicExch(flag, 1); return; }
-    for (int64_t p0 = r0 + sub; p0 < r1; p0 += 4 * nsub) {
-        int32_t tg[4], slot[4];
-        double tt[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (p0 + u * nsub < r1) { tg[u] = __ldg(a.stgt + p0 + u * nsub); tt[u] = __ldg(ob.term_src + p0 + u * nsub); }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (p0 + u * nsub < r1) slot[u] = atomicAdd(cnt + tg[u] / kSynBin, 1);
+// the events of source i (relative to the object's range) of step slot `now`
+// (step mod ring) into the bins: of records [r0, r1), every `stride`-th from the
+// lane's own on, four at a time (loads, then slots, then stores); only those of
+// delay dmin or more
+__device__ __forceinline__ void synp_push(const SynPersistArgs &a, const SynRec *rec, int64_t i, int64_t r0, int64_t r1, int now,
+                                          int lane, int stride, int dmin) {
+    for (int64_t p0 = r0 + lane; p0 < r1; p0 += 4 * stride) {
+        SynRec v[4];
+        int at[4], slot[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int64_t p = p0 + u * nsub;
-            if (p >= r1) break;
-            if (slot[u] >= kSynBinCap) { atomicExch(flag, 1); continue; }
-            const int64_t j = tg[u];
-            const int64_t e = (j / kSynBin) * kSynBinCap + slot[u];
-            key[e] = ((unsigned long long)(j * 4 + k) << 40) | ((unsigned long long)(255 - d) << 32) |
-                     ((unsigned long long)i << 8) | (unsigned long long)(p - r0);
-            tv[e] = tt[u];
+            at[u] = -1;
+            if (p0 + u * stride < r1) v[u] = __ldg(rec + p0 + u * stride);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (p0 + u * stride < r1) {
+                const int d = 255 - (int)((v[u].x >> 44) & 255u);
+                if (d < dmin) continue;
+                int row = now + d;
+                row -= row >= a.ring ? a.ring : 0;
+                at[u] = row * a.nbins + (int)((v[u].x >> 20) & 0xffffffu);
+                slot[u] = atomicAdd(a.bin_cnt + at[u], 1);
+            }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (at[u] < 0) continue;
+            if (slot[u] >= a.cap) continue;              // (the count tells)
+            v[u].x = (v[u].x & ~(0xffffffull << 20)) | ((unsigned long long)i << 20);
+            __stcg(a.bin_ev + (int64_t)at[u] * a.cap + slot[u], v[u]);
+        }
+    }
+}
+
+// the records of an object's synapses (a warp per source)
+static __global__ void __launch_bounds__(256) k_synp_records(const SynEvArgs e, int k, SynRec *rec) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x / 32);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); i < e.sn; i += nw) {
+        const int64_t r0 = e.srcptr[i], r1 = e.srcptr[i + 1];
+        for (int64_t p = r0 + lane; p < r1; p += 32) {
+            const unsigned long long j = (unsigned long long)e.stgt[p];
+            SynRec v;
+            v.x = ((j % kSynBin) << 54) | ((unsigned long long)k << 52) | ((unsigned long long)(255 - e.sd[p]) << 44) |
+                  ((j / kSynBin) << 20) | (unsigned long long)(p - r0);
+            v.y = (unsigned long long)__double_as_longlong(e.term[e.sq[p]]);
+            rec[p] = v;
+        }
+    }
+}
+
+// the (emptied) ring filled with the events still to come of the spikes in the
+// history: blocks of one object's (step back, word) pairs, a warp per pair
+static __global__ void __launch_bounds__(256) k_synp_refill(const __grid_constant__ SynPersistArgs a, int k) {
+    const SynEvArgs &e = a.o[k].e;
+    const long long nstep = a.ctl->nstep;
+    const int lane = threadIdx.x & 31;
+    const int64_t w0 = e.so >> 5, nw = ((e.so + e.sn + 31) >> 5) - w0;
+    for (int64_t x = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5); x < nw * e.dmax;
+         x += (int64_t)gridDim.x * (blockDim.x / 32)) {
+        const int back = 1 + (int)(x / nw);
+        const int64_t wi = w0 + x % nw;
+        if (nstep < back) continue;
+        uint32_t word = masked_word(a.hist + (int64_t)(((int)nstep - back) % a.depth) * a.nwords, wi, e.so, e.so + e.sn);
+        for (; word; word &= word - 1) {
+            const int64_t i = (wi << 5) + (__ffs(word) - 1) - e.so;
+            synp_push(a, a.o[k].rec, i, e.srcptr[i], e.srcptr[i + 1], (int)((nstep - back) % a.ring), lane, 32, back);
         }
     }
 }
@@ -109,27 +158,26 @@ __device__ __forceinline__ void synp_apply(const SynPersistArgs &a, double (&s)[
         if (uu == u) uset<double, NV>(s[uu], v, sub ? __dsub_rn(uget<double, NV>(s[uu], v), t) : __dadd_rn(uget<double, NV>(s[uu], v), t));
 }
 
-// C(t) for this block's bin (block-uniform call; synchronises)
+// C(t) for this block's bin (block-uniform call; synchronises).  tcnt is zero
+// and `over` false at entry, and again on return.
 template <int NV>
-__device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, int par, bool pull,
-                                          double (&s)[kSPNpt][NV]) {
-    extern __shared__ unsigned char syn_smem[];
-    unsigned long long *key = reinterpret_cast<unsigned long long *>(syn_smem);
+__device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, int now,
+                                          double (&s)[kSPNpt][NV], int (&tcnt)[kSynBin], int &over) {
+    extern __shared__ __align__(16) unsigned char syn_smem[];
+    SynRec *tab = reinterpret_cast<SynRec *>(syn_smem);                          // [kSPTab][kSPBn]
+    unsigned long long *key = reinterpret_cast<unsigned long long *>(syn_smem);  // or the bin in order
     double *tv = reinterpret_cast<double *>(key + kSynBinCap);
-    __shared__ int tcnt[kSynBin];
     __shared__ int wsum[kSPTh / 32], maxc;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int bin = (int)blockIdx.x - a.blk0;
     if (bin < 0 || bin >= a.nbins) return;
     const int64_t jb = (int64_t)bin * kSynBin;
-    int *cnt = a.bin_cnt + (int64_t)par * a.nbins + bin;
-    const unsigned long long *gkey = a.bin_key + ((int64_t)par * a.nbins + bin) * kSynBinCap;
-    const double *gt = a.bin_t + ((int64_t)par * a.nbins + bin) * kSynBinCap;
+    int *cnt = a.bin_cnt + now * a.nbins + bin;
+    const SynRec *gev = a.bin_ev + ((int64_t)now * a.nbins + bin) * a.cap;
     // the first kSPTh entries loaded beside the count (those beyond it unused)
-    const unsigned long long k0 = __ldcg(gkey + tid);
-    const double t0v = __ldcg(gt + tid);
-    const int n = min(__ldcg(cnt), kSynBinCap);
-    if (pull) {
+    const SynRec e0 = __ldcg(gev + tid);
+    const int n = __ldcg(cnt);
+    if (n > a.cap) {
         // the pull's test for every target of the bin, object by object
         const int row0 = (int)t % a.depth;
 #pragma unroll
@@ -151,13 +199,36 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
             }
         }
     } else if (n > 0) {
-#pragma unroll
-        for (int u = 0; u < kSPNpt; ++u) tcnt[u * kSPTh + tid] = 0;
-        if (tid == 0) maxc = 0;
+        // each event beside the others of its target, in the order of arrival
+        for (int e = tid; e < n; e += kSPTh) {
+            const SynRec v = e == tid ? e0 : __ldcg(gev + e);
+            const int j = (int)(v.x >> 54);
+            const int pos = atomicAdd(&tcnt[j], 1);
+            if (pos < kSPTab) tab[pos * kSPBn + j] = v;
+            else over = 1;
+        }
         __syncthreads();
-        if (tid < n) atomicAdd(&tcnt[(int)((k0 >> 42) - (unsigned long long)jb)], 1);
-        for (int e = tid + kSPTh; e < n; e += kSPTh)
-            atomicAdd(&tcnt[(int)((__ldcg(gkey + e) >> 42) - (unsigned long long)jb)], 1);
+        if (!over) {                                             // uniform
+            // a target's few events by ascending key
+#pragma unroll
+            for (int u = 0; u < kSPNpt; ++u) {
+                const int j = u * kSPTh + tid, c = tcnt[j];
+                if (!c) continue;
+                tcnt[j] = 0;
+                unsigned long long from = 0;
+                for (int r = 0; r < c; ++r) {
+                    SynRec best = tab[j];
+                    bool have = best.x >= from;
+                    for (int q = 1; q < c; ++q) {
+                        const SynRec v = tab[q * kSPBn + j];
+                        if (v.x >= from && (!have || v.x < best.x)) { best = v; have = true; }
+                    }
+                    synp_apply<NV>(a, s, u, (int)((best.x >> 52) & 3u), __longlong_as_double((long long)best.y));
+                    from = best.x + 1;
+                }
+            }
+        } else {
+        if (tid == 0) maxc = 0;
         __syncthreads();
         int cu[kSPNpt], c = 0, cmax = 0;
 #pragma unroll
@@ -183,16 +254,11 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
                 for (int u = 0; u < kSPNpt; ++u) { tcnt[u * kSPTh + tid] = b; b += cu[u]; }
             }
             __syncthreads();
-            if (tid < n) {
-                const int pos = atomicAdd(&tcnt[(int)((k0 >> 42) - (unsigned long long)jb)], 1);
-                key[pos] = k0;
-                tv[pos] = t0v;
-            }
-            for (int e = tid + kSPTh; e < n; e += kSPTh) {
-                const unsigned long long kk = __ldcg(gkey + e);
-                const int pos = atomicAdd(&tcnt[(int)((kk >> 42) - (unsigned long long)jb)], 1);
-                key[pos] = kk;
-                tv[pos] = __ldcg(gt + e);
+            for (int e = tid; e < n; e += kSPTh) {
+                const SynRec v = e == tid ? e0 : __ldcg(gev + e);
+                const int pos = atomicAdd(&tcnt[(int)(v.x >> 54)], 1);
+                key[pos] = v.x;
+                tv[pos] = __longlong_as_double((long long)v.y);
             }
             __syncthreads();
             int sb = beg;
@@ -208,7 +274,7 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
                         key[w + 1] = kk;
                         tv[w + 1] = tt;
                     }
-                    for (int e = sb; e < sb + cc; ++e) synp_apply<NV>(a, s, u, (int)((key[e] >> 40) & 3u), tv[e]);
+                    for (int e = sb; e < sb + cc; ++e) synp_apply<NV>(a, s, u, (int)((key[e] >> 52) & 3u), tv[e]);
                 }
                 sb += cc;
             }
@@ -216,7 +282,7 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
             int m = 1;
             while (m < n) m <<= 1;
             for (int e = tid; e < m; e += kSPTh) {
-                if (e < n) { key[e] = __ldcg(gkey + e); tv[e] = __ldcg(gt + e); }
+                if (e < n) { const SynRec v = __ldcg(gev + e); key[e] = v.x; tv[e] = __longlong_as_double((long long)v.y); }
                 else { key[e] = ~0ull; tv[e] = 0.0; }
             }
             __syncthreads();
@@ -239,30 +305,52 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
 #pragma unroll
             for (int u = 0; u < kSPNpt; ++u) {
                 if (!cu[u]) continue;
-                const unsigned long long want = (unsigned long long)(jb + u * kSPTh + tid);
+                const unsigned long long want = (unsigned long long)(u * kSPTh + tid);
                 int l = 0, h = n;
-                while (l < h) { const int mm = (l + h) >> 1; if ((key[mm] >> 42) < want) l = mm + 1; else h = mm; }
-                for (int e = l; e < n && (key[e] >> 42) == want; ++e)
-                    synp_apply<NV>(a, s, u, (int)((key[e] >> 40) & 3u), tv[e]);
+                while (l < h) { const int mm = (l + h) >> 1; if ((key[mm] >> 54) < want) l = mm + 1; else h = mm; }
+                for (int e = l; e < n && (key[e] >> 54) == want; ++e)
+                    synp_apply<NV>(a, s, u, (int)((key[e] >> 52) & 3u), tv[e]);
             }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < kSPNpt; ++u) tcnt[u * kSPTh + tid] = 0;
         }
     }
     __syncthreads();                     // every thread has read the count; shared memory free
-    if (tid == 0) *cnt = 0;              // pushed into again in A(t+2)
+    if (tid == 0) { *cnt = 0; over = 0; }    // (the slot is pushed into again in A(t+3))
 }
 
 template <int NV, bool DIAG>
 __global__ void __launch_bounds__(kSPTh, 2) k_syn_persist(const __grid_constant__ SynPersistArgs a) {
-    __shared__ uint32_t words[kSPBn / 32];
-    __shared__ int abort_flag, pull_s;
+    extern __shared__ __align__(16) unsigned char syn_smem[];
+    // row starts of the block's neurons as sources, relative to the first one's
+    uint32_t *rows = reinterpret_cast<uint32_t *>(syn_smem + (size_t)kSynBinCap * sizeof(SynRec));   // [nobj][kSPBn + 1]
+    __shared__ int64_t row0[kSynEvMerge];
+    __shared__ uint16_t fired[kSPBn];            // the step's spikes, and how many
+    __shared__ int nfired;
+    __shared__ int tcnt[kSynBin], over;          // synp_bins
+    __shared__ int abort_flag;
     __shared__ double stash[kSPBn];              // StateMonitor values of the block's neurons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int base = blockIdx.x * kSPBn;         // neuron counts < 2^31
     const int nvalid = (int)min((int64_t)kSPBn, a.n - (int64_t)base);
     const unsigned int G = gridDim.x;
     const long long t0 = a.ctl->nstep;          // step counters are below 2^31 (checked by the host)
-    const int nl = kSPTh - 32 * a.nobj;          // threads on the spike lists; the rest on this step's words
-    if (tid == 0) abort_flag = 0;
+    if (tid == 0) { abort_flag = 0; nfired = 0; over = 0; }
+#pragma unroll
+    for (int u = 0; u < kSPNpt; ++u) tcnt[u * kSPTh + tid] = 0;
+    for (int k = 0; k < a.nobj; ++k) {
+        const SynEvArgs &e = a.o[k].e;
+        auto start = [&](int64_t li) {           // (neurons outside the object's sources have empty rows)
+            const int64_t i = (int64_t)base + li - e.so;
+            return e.srcptr[i < 0 ? 0 : (i > e.sn ? e.sn : i)];
+        };
+        const int64_t r0 = start(0);
+        if (tid == 0) row0[k] = r0;
+        for (int li = tid; li <= kSPBn; li += kSPTh) rows[k * (kSPBn + 1) + li] = (uint32_t)(start(li) - r0);
+    }
+    int now = (int)(t0 % a.ring);                // the step's slot
     double s[kSPNpt][NV];
 #pragma unroll
     for (int u = 0; u < kSPNpt; ++u) {
@@ -273,9 +361,8 @@ __global__ void __launch_bounds__(kSPTh, 2) k_syn_persist(const __grid_constant_
     unsigned long long my_spikes = 0;
     __syncthreads();
 
-    for (int st = 0; st < a.nsteps; ++st) {
+    for (int st = 0; st < a.nsteps; ++st, now = now + 1 == a.ring ? 0 : now + 1) {
         const long long t = t0 + st;
-        const int par = (int)(t & 1);
         // ---- A(t): update (x = A s + C, the order of linear_row), threshold
         {
             double x[kSPNpt][NV];
@@ -326,66 +413,29 @@ __global__ void __launch_bounds__(kSPTh, 2) k_syn_persist(const __grid_constant_
             spk = spk && li < nvalid;
             spk_bits |= (spk ? 1u : 0u) << u;
             const uint32_t ball = __ballot_sync(0xffffffffu, spk);
+            if (ball) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&nfired, __popc(ball));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (spk) fired[at + __popc(ball & ((1u << lane) - 1u))] = (uint16_t)li;
+            }
             if (lane == 0) {
                 const int w = u * (kSPTh / 32) + warp;
-                words[w] = ball;
                 a.hist[(int64_t)((int)t % a.depth) * a.nwords + (base >> 5) + w] = ball;
                 if (a.mon_words) a.mon_words[(int64_t)st * a.mon_stride + (base >> 5) + w] = ball;
                 my_spikes += __popc(ball);
             }
         }
         __syncthreads();
-        if (blockIdx.x == 0) {
-            if (tid < a.nobj) {
-                const SynEvArgs &e = a.o[tid].e;
-                e.scnt[((int)t + 1) % e.sdepth] = 0;              // step t+1's list starts empty
-            }
-            if (tid == 32) a.use_pull[((int)t + 1) % 3] = 0;     // step t+1's overflow flag (last read in C(t-2))
-        }
-        int *flag = a.use_pull + (int)t % 3;
-        int *bcnt = a.bin_cnt + (int64_t)par * a.nbins;
-        unsigned long long *bkey = a.bin_key + (int64_t)par * a.nbins * kSynBinCap;
-        double *bt = a.bin_t + (int64_t)par * a.nbins * kSynBinCap;
-        if (tid >= nl) {
-            // this block's spikes: into object k's list of step t (when they
-            // are its sources), with their delay-0 events
-            const int k = (tid - nl) >> 5, w = tid & 31;
-            const SynPersistObj &ob = a.o[k];
-            const SynEvArgs &e = ob.e;
-            const int64_t wb = (int64_t)((base >> 5) + w) << 5;
-            uint32_t word = words[w];
-            if (wb < e.so) { const int sh = (int)(e.so - wb); word = sh >= 32 ? 0u : (word & (0xffffffffu << sh)); }
-            if (wb + 32 > e.so + e.sn) { const int keep = (int)(e.so + e.sn - wb); word = keep <= 0 ? 0u : (keep >= 32 ? word : (word & ((1u << keep) - 1u))); }
-            if (word) {
-                const int row = (int)t % e.sdepth;
-                const int pos = atomicAdd(e.scnt + row, __popc(word));   // used after the pushes
-                for (uint32_t wv = word; wv; wv &= wv - 1)
-                    synp_push(ob, k, wb + (__ffs(wv) - 1) - e.so, 0, 0, 1, flag, bcnt, bkey, bt);
-                int32_t *L = e.slist + (int64_t)row * e.sn + pos;
-                for (uint32_t wv = word; wv; wv &= wv - 1) *L++ = (int32_t)(wb + (__ffs(wv) - 1) - e.so);
-            }
-        } else {
-            // the spike lists of steps t-1 .. t-dmax dealt out over the blocks
-            for (int pr = blockIdx.x; pr < a.pair0[a.nobj] * a.nparts; pr += G) {
-                const int pair = pr / a.nparts, part = pr % a.nparts;
-                int k = 0;
-                while (k + 1 < a.nobj && pair >= a.pair0[k + 1]) ++k;
-                const SynPersistObj &ob = a.o[k];
-                const SynEvArgs &e = ob.e;
-                const int d = 1 + pair - a.pair0[k];
-                if (t < d) continue;
-                const int row = ((int)t - d) % e.sdepth;
-                const int32_t *L = e.slist + (int64_t)row * e.sn;
-                // kSynSub threads per listed source, each with a share of its synapses
-                const int q0 = (part * nl + tid) / kSynSub, sub = tid % kSynSub;
-                const int32_t first = q0 < e.sn ? __ldcg(L + q0) : 0;   // loaded beside the count
-                const int cnt = __ldcg(e.scnt + row);
-                for (int q = q0; q < cnt; q += a.nparts * nl / kSynSub)
-                    synp_push(ob, k, q == q0 ? first : __ldcg(L + q), d, sub, kSynSub, flag, bcnt, bkey, bt);
-            }
+        for (int q = warp; q < nfired * a.nobj * kSPParts; q += kSPTh / 32) {
+            const int part = q % kSPParts, qo = q / kSPParts, k = qo % a.nobj, li = fired[qo / a.nobj];
+            const uint32_t *rw = rows + k * (kSPBn + 1) + li;
+            synp_push(a, a.o[k].rec, (int64_t)base + li - a.o[k].e.so, row0[k] + rw[0], row0[k] + rw[1], now, part * 32 + lane,
+                      32 * kSPParts, 0);
         }
         // ---- arrive at step t; wait for every block's arrival
         __syncthreads();
+        if (tid == 0) nfired = 0;
         if (tid == 0 && (int)blockIdx.x != a.hold_block) red_release_add(a.arrived + (st & 3), 1u);
         if (tid == 32) {
             const unsigned int *ctr = a.arrived + (st & 3);
@@ -395,14 +445,11 @@ __global__ void __launch_bounds__(kSPTh, 2) k_syn_persist(const __grid_constant_
                 if (++it > a.spin_limit) { abort_flag = 1; bg_raise(a.ctl, BG_DERR_TIMEOUT, t); break; }
                 __nanosleep(32);
             }
-            // the step's overflow flag, read once per block (every warp of
-            // every block reading one address queues at one L2 slice)
-            pull_s = __ldcg(flag);
         }
         __syncthreads();
         if (abort_flag) break;
         // ---- C(t): this block's bin, then the resets of step t
-        synp_bins<NV>(a, t, par, pull_s != 0, s);
+        synp_bins<NV>(a, t, now, s, tcnt, over);
         if (a.reset_kind == 1) {
 #pragma unroll
             for (int u = 0; u < kSPNpt; ++u)
@@ -435,12 +482,6 @@ __global__ void __launch_bounds__(kSPTh, 2) k_syn_persist(const __grid_constant_
         }
     }
     block_count(a.spikes, my_spikes);
-}
-
-// the statement's term per synapse in by-source order: out[p] = term[sq[p]]
-static __global__ void k_syn_term_src(const int32_t *sq, const double *term, int64_t nsyn, double *out) {
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nsyn; p += (int64_t)gridDim.x * blockDim.x)
-        out[p] = term[sq[p]];
 }
 
 }  // namespace bg
