@@ -1523,6 +1523,17 @@ int build_persist(bg_net *net) {
             q.packed = c.dPacked;
         }
     }
+    {
+        int64_t row = 0;                                     // the longest average row of the connections
+        bool packed = true;
+        for (int p = 0; p < a.npush; ++p) {
+            const HConn &c = net->conns[p];
+            packed = packed && (a.push[p].packed || c.nnz == 0);
+            row = std::max(row, c.nnz / std::max<int64_t>(1, c.sn));
+        }
+        a.lparts = packed ? 0 : -1;
+        while (a.lparts >= 0 && a.lparts < 4 && ((int64_t)128 << a.lparts) < row) ++a.lparts;
+    }
     a.spikes = net->dCounters;
     a.arrived = net->dArrived;
     a.lag = min_d >= 1 ? 2 : 1;

@@ -40,6 +40,10 @@ template <typename T> struct PersistArgs {
     unsigned int *arrived;      // [4] arrivals per step mod 4 (zeroed before the launch)
     int nsteps;
     int lag;                    // 1 when some delay is zero, else 2
+    // pushes of packed synapses: 2^lparts warps take a spike's row (four synapses a
+    // lane in flight cover a row of average length); -1 when some push is not
+    // packed: all threads take batches of spikes' rows, flattened
+    int lparts;
     uint32_t *mon_words;        // spike monitors: spike words of each step of the launch, else null
     int64_t mon_stride;         // words per step in mon_words
     unsigned int spin_limit;    // polls of a wait before it gives up (BG_DERR_TIMEOUT)
@@ -78,6 +82,7 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
     __shared__ int64_t srow1[kPersistMaxPush][kPushBatch];      // first batch, per connection
     __shared__ int32_t spref1[kPersistMaxPush][kPushBatch + 1];
     __shared__ int nsp, abort_flag;
+    __shared__ int nfired[2];                    // spikes of the block's step, by parity (listed in sl)
     __shared__ T stash[BN];                      // StateMonitor values of the block's neurons
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int base = blockIdx.x * BN;               // neuron counts < 2^31
@@ -94,7 +99,7 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
         }
         if (tid == 0) srp0[p] = q.rowptr[r0];
     }
-    if (tid == 0) abort_flag = 0;
+    if (tid == 0) { abort_flag = 0; nfired[0] = nfired[1] = 0; }
     // deliveries: which of this thread's neurons each one targets (bit u),
     // the thread's column in ring row 0, and the row delivered next (ring
     // rows advance by one per step: no division in the loop)
@@ -287,6 +292,12 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
             spk[u] = spk[u] && li < nvalid;
             prev_spk |= (spk[u] ? 1u : 0u) << u;
             const uint32_t ball = __ballot_sync(0xffffffffu, spk[u]);
+            if (ball && a.lparts >= 0) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&nfired[st & 1], __popc(ball));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (spk[u]) sl[at + __popc(ball & ((1u << lane) - 1u))] = li;
+            }
             // (no history words: nothing reads them on this path)
             if (lane == 0) {
                 words[u * (TH / 32) + warp] = ball;
@@ -297,9 +308,46 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
         const int any_spike = __syncthreads_or(prev_spk != 0);
         // spike monitors: the block's words of this step, one coalesced row
         if (a.mon_words && tid < BN / 32) a.mon_words[(int64_t)st * a.mon_stride + (base >> 5) + tid] = words[tid];
-        // ---- push this block's spikes: one flattened scatter over every
+        if (tid == 0) nfired[(st + 1) & 1] = 0;
+        // ---- push this block's spikes, in any order (counts): a few warps per
+        // spike straight from its row.  (One warp listing the spikes in order and
+        // scanning their row lengths for a flattened scatter put about 600
+        // cycles and a barrier into every step with a spike: 262144 neurons of in-degree
+        // 1000, 3.77 -> 3.42 us a step; 60000 of 600, 2.84 -> 2.58.)
+        if (a.lparts >= 0 && any_spike) {
+            const int nw = nfired[st & 1] << a.lparts;
+            for (int q = warp; q < nw; q += TH / 32) {
+                const int j = sl[q >> a.lparts], part = q & ((1 << a.lparts) - 1);
+#pragma unroll
+                for (int p = 0; p < kPersistMaxPush; ++p) {
+                    if (p >= a.npush) break;
+                    if (!pact[p]) continue;
+                    const uint32_t r0 = srp[p][j], r1 = srp[p][j + 1];
+                    if (part == 0 && lane == 0) my_events[p] += (unsigned long long)(r1 - r0);
+                    const Push<T> &Q = a.push[p];
+                    const uint32_t *pk0 = Q.packed + srp0[p];
+                    const uint32_t stride = 32u << a.lparts;
+                    // (64-bit: a row may end just below 2^32)
+                    for (int64_t e = (int64_t)r0 + part * 32 + lane; e < (int64_t)r1; e += 4 * (int64_t)stride) {
+                        uint32_t v[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            v[u] = 0xffffffffu;
+                            if (e + u * (int64_t)stride < (int64_t)r1) v[u] = __ldg(pk0 + e + u * (int64_t)stride);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (v[u] == 0xffffffffu) continue;
+                            const int row = pcur[p] + (int)(v[u] >> 24);
+                            cring_add(Q.cring + (int64_t)(row >= Q.md ? row - Q.md : row) * Q.tnp, (int32_t)(v[u] & 0xffffffu));
+                        }
+                    }
+                }
+            }
+        }
+        // ---- some push not packed: one flattened scatter over every
         // (connection, spike) pair of the block
-        if (a.npush && any_spike) {
+        if (a.lparts < 0 && a.npush && any_spike) {
             // warp 0: the spike list, then for every connection the row starts
             // and an inclusive scan of the row lengths of a batch of spikes
             // (the first batch here, before the barrier; later ones below)
@@ -360,8 +408,7 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
                     }
                     const int total = pref[nb];
                     if (tid == 0) my_events[p] += (unsigned long long)total;
-                    if (q.packed) scatter_batch_packed<TH>(q.packed, q.cring, q.tnp, q.md, cur, rows, pref, nb, total);
-                    else scatter_batch<T, TH>(q, cur, rows, pref, nb, total);
+                    scatter_batch<T, TH>(q, cur, rows, pref, nb, total);
                 }
             }
         }
@@ -383,7 +430,7 @@ __global__ void __launch_bounds__(TH, TH <= 512 ? 2 : 1) k_persist(const Persist
         }
     }
     block_count(a.spikes, my_spikes);
-    if (tid == 0)
+    if (lane == 0)
         for (int p = 0; p < a.npush; ++p)
             if (my_events[p] && a.push[p].events) atomicAdd(a.push[p].events, my_events[p]);
 }
