@@ -588,7 +588,7 @@ int build_stdp_step(bg_net *net, int cid) {
     const int64_t bands = (c.sn + bg::kFlushRows - 1) / bg::kFlushRows;
     const unsigned fgrid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(bands, (int64_t)sm_count() * 8));
     const float flo = (float)s.wmin, fhi = (float)s.wmax;
-    const bool fast = s.post_mode == 0 && sizeof(WT) == 4 && flo >= 0.0f && flo <= fhi;
+    const bool fast = s.post_mode == 0 && sizeof(WT) == 4 && flo >= 0.0f && !std::signbit(flo) && std::isfinite(flo) && flo <= fhi;   // (lazy_update)
     net->flushes.push_back([f, fgrid, fast](cudaStream_t st) {
         if (fast) bg::k_stdp_flush<WT, true><<<fgrid, bg::kFlushThreads, 0, st>>>(f);
         else bg::k_stdp_flush<WT, false><<<fgrid, bg::kFlushThreads, 0, st>>>(f);

@@ -54,11 +54,21 @@ template <typename T> struct StdpStepArgs {
 };
 
 // One postsynaptic update of a weight, as stdp_w_val.  FAST (additive, FP32
-// weights, 0 <= lo <= hi, w >= 0 and not NaN): the weight's bits placed in a
-// double are w * 2^-896 exactly (zeros and subnormals too), so one FMA gives
-// w + add with the one rounding of the double sum, where widening w takes a
-// conversion on a pipe a quarter as wide as the FP64 one; the clip is a
-// minimum and a maximum (its sign of a zero aside the same).
+// weights, bounds 0 <= lo <= hi with lo finite and not -0): the weight's bits
+// placed in a double are w * 2^-896 exactly (zeros and subnormals too), so one
+// FMA gives w + add with the one rounding of the double sum, where widening w
+// takes a conversion on a pipe a quarter as wide as the FP64 one; the clip is a
+// minimum and a maximum.  Both hold for lazy_plain_weight and lazy_plain_add
+// only:
+//  - a weight with its sign bit set (-0 among them), infinite or NaN is another
+//    number in that place;
+//  - a NaN sum would leave a minimum and maximum as a bound, where the
+//    comparisons of stdp_w_val keep it; weights below 2^120 and additions of at
+//    most 2^100 make no infinity in kLazySteps additions either;
+//  - a sum that rounds to -0 would leave them as +0.  A weight >= 0 gets there
+//    by a negative addition of at most 2^-96 only: past that it must cancel a
+//    weight above 2^-97, and the sum is then a multiple of 2^-148, which is 0
+//    (+0) or too large to round to zero.
 template <typename WT, bool FAST>
 __device__ __forceinline__ WT lazy_update(WT w, double add, float flo, float fhi, double wmin, double wmax, int mode, double wx) {
     if constexpr (FAST && sizeof(WT) == 4) {
@@ -68,6 +78,11 @@ __device__ __forceinline__ WT lazy_update(WT w, double add, float flo, float fhi
     } else {
         return stdp_w_val<WT>(w, add, wmin, wmax, mode, wx);
     }
+}
+__device__ __forceinline__ bool lazy_plain_weight(float w) { return __float_as_uint(w) < 0x7b800000u; }   // +0 <= w < 2^120
+__device__ __forceinline__ bool lazy_plain_add(double add) {
+    const double m = fabs(add);
+    return m <= 0x1p100 && !(__double2hiint(add) < 0 && m <= 0x1p-96);
 }
 
 __device__ __forceinline__ bool spike_bit(const uint32_t *H, int64_t i) { return (H[i >> 5] >> (i & 31)) & 1u; }
@@ -198,14 +213,15 @@ struct StdpFlushArgs {
 };
 
 // Applies every pending update to the whole matrix.  A block takes bands of
-// kFlushRows rows: their trace records go to shared memory (0 for the steps a
-// row has taken already: such a row was clipped by its presynaptic update
-// since, so adding 0 leaves it as it is), then a thread takes one column of
-// the band at a time and walks the column's spikes, all rows of the band side
-// by side.  Warps whose 32 columns have no spikes skip them.
+// kFlushRows rows: their trace records go to shared memory, with -0 for the
+// steps a row has taken already (w + -0 is w, and such a row was clipped by its
+// presynaptic update since; the general form skips them), then a thread takes
+// one column of the band at a time and walks the column's spikes, all rows of
+// the band side by side.  Warps whose 32 columns have no spikes skip them.
 template <typename WT, bool FAST>
 __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArgs a) {
     __shared__ double tab[kFlushRows][kLazySteps];
+    __shared__ int from[kFlushRows];               // first step a row has not taken
     const int tid = threadIdx.x;
     const int n = (int)(a.ctl->nstep - a.lz->base), win = a.lz->win;
     const unsigned long long *rowmask = a.rowmask + (int64_t)win * a.sn, *colmask = a.colmask + (int64_t)win * a.tn;
@@ -220,27 +236,31 @@ __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArg
     for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
         const int64_t i0 = b * kFlushRows;
         const int rows = (int)min((int64_t)kFlushRows, a.sn - i0);
+        int fits = 1;                              // the band's additions keep the fast form exact
         for (int k = tid; k < kFlushRows * kLazySteps; k += kFlushThreads) {
             const int r = k / kLazySteps, s = k % kLazySteps;
-            double x = 0.0;
-            if (r < rows && s < n) {
-                const unsigned long long rm = rowmask[i0 + r];
-                if (!rm || s >= 63 - __clzll((long long)rm)) x = a.rec[(i0 + r) * kLazySteps + s];
+            const unsigned long long rm = r < rows ? rowmask[i0 + r] : 0ull;
+            const int lo = r >= rows ? kLazySteps : (rm ? 63 - __clzll((long long)rm) : 0);
+            if (s == 0) from[r] = lo;
+            double x = -0.0;
+            if (s >= lo && s < n) {
+                x = a.rec[(i0 + r) * kLazySteps + s];
+                fits &= FAST && lazy_plain_add(x);
             }
             tab[r][s] = x;
         }
-        __syncthreads();
+        const bool band = __syncthreads_and(fits) != 0;
         for (int64_t c0 = 0; c0 < a.tn; c0 += kFlushThreads) {
             const int64_t j = c0 + tid;
             unsigned long long m = j < a.tn ? colmask[j] : 0ull;
             if (!__any_sync(0xffffffffu, m != 0ull)) continue;
             if (!m) continue;
             WT w[kFlushRows];
-            bool plain = FAST;                     // every weight here is >= 0 (and none NaN)
+            bool plain = FAST && band;
 #pragma unroll
             for (int r = 0; r < kFlushRows; ++r) {
                 w[r] = r < rows ? W[(i0 + r) * a.tn + j] : WT(0);
-                plain = plain && w[r] >= WT(0);
+                plain = plain && lazy_plain_weight((float)w[r]);
             }
             if (plain) {
                 do {
@@ -256,7 +276,7 @@ __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArg
                     m &= m - 1;
 #pragma unroll
                     for (int r = 0; r < kFlushRows; ++r)
-                        w[r] = lazy_update<WT, false>(w[r], tab[r][s], flo, fhi, a.wmin, a.wmax, a.mode, a.wx);
+                        if (s >= from[r]) w[r] = lazy_update<WT, false>(w[r], tab[r][s], flo, fhi, a.wmin, a.wmax, a.mode, a.wx);
                 } while (m);
             }
 #pragma unroll
