@@ -1453,7 +1453,7 @@ int build_persist(bg_net *net) {
             const int64_t hi = std::min(std::max((b + 1) * bn - c.so, (int64_t)0), c.sn);
             if (c.rowptr[hi] - c.rowptr[lo] >= ((int64_t)1 << 32)) return BG_OK;
         }
-    if (!cluster && net->alloc(&net->dArrived, 64) != cudaSuccess) return fail(BG_ENOMEM, "arrival counter");
+    if (!cluster && !net->dArrived && net->alloc(&net->dArrived, 64) != cudaSuccess) return fail(BG_ENOMEM, "arrival counter");
     bg::PersistArgs<T> a;
     std::memset(&a, 0, sizeof(a));
     a.ctl = net->dCtl; a.S = (T *)g.dS; a.n = g.n; a.npad = g.npad; a.useC = g.useC;
@@ -1469,16 +1469,18 @@ int build_persist(bg_net *net) {
     // in row t mod 3, delivered at the top of step t+1; blocks are at most
     // one step apart) and the table {0, w}
     for (HConn &c : net->conns) {
-        if (cluster || !persist_direct(c) || c.dDirRing) continue;
+        if (cluster || !persist_direct(c)) continue;
         int st = c.dir_kmax < 0 ? max_indegree(net, c, &c.dir_kmax) : BG_OK;
         if (st) return st;
         if (c.dir_kmax >= 65535) return BG_OK;               // 16-bit counts
-        c.dir_md = 3;
-        c.tnp = (c.tn + 1) & ~1ll;
-        if (net->alloc(&c.dDirRing, (size_t)c.dir_md * c.tnp * 2) != cudaSuccess ||
-            net->alloc(&c.dDirTable, 2 * sizeof(T)) != cudaSuccess)
-            return fail(BG_ENOMEM, "count ring");
-        BG_CUDA(cudaMemsetAsync(c.dDirRing, 0, (size_t)c.dir_md * c.tnp * 2, net->stream));
+        if (!c.dDirRing) {
+            c.dir_md = 3;
+            c.tnp = (c.tn + 1) & ~1ll;
+            if (net->alloc(&c.dDirRing, (size_t)c.dir_md * c.tnp * 2) != cudaSuccess ||
+                net->alloc(&c.dDirTable, 2 * sizeof(T)) != cudaSuccess)
+                return fail(BG_ENOMEM, "count ring");
+            BG_CUDA(cudaMemsetAsync(c.dDirRing, 0, (size_t)c.dir_md * c.tnp * 2, net->stream));
+        }
         const double w0 = c.w_bits == 64 ? *(const double *)c.w.data() : (double)*(const float *)c.w.data();
         const T tab[2] = {T(0), (T)w0};
         st = upload(net, c.dDirTable, tab, sizeof(tab));
@@ -2153,6 +2155,8 @@ int bg_conn_read_weights(bg_net *n, int32_t cid, void *out, int64_t bytes) {
     return BG_OK;
 }
 
+static int build_launches(bg_net *n);
+
 int bg_conn_set_weights(bg_net *n, int32_t cid, const double *in) {
     if (!n || cid < 0 || cid >= (int32_t)n->conns.size() || !in) return fail(BG_EINVAL, "bg_conn_set_weights");
     HConn &c = n->conns[cid];
@@ -2180,8 +2184,22 @@ int bg_conn_set_weights(bg_net *n, int32_t cid, const double *in) {
         else ((float *)c.w.data())[k] = (float)in[k];
     }
     if (n->prepared) {
+        BG_CUDA(cudaSetDevice(n->device));
         BG_CUDA(cudaStreamSynchronize(n->stream));
         BG_CUDA(cudaMemcpy(c.dW, c.w.data(), c.w.size(), cudaMemcpyHostToDevice));
+        if (!c.hetero && !c.dense && c.mod_var < 0 && c.stdp < 0) {
+            // the persistent launches hold a shared weight's value, and a
+            // stepped one adds in an order only where the weights differ
+            const int64_t wb = c.w_bits / 8;
+            bool same = true;
+            for (int64_t k = 1; k < cnt; ++k) same = same && std::memcmp(c.w.data() + k * wb, c.w.data(), wb) == 0;
+            if (same != c.homogeneous || (same && n->persist)) {
+                c.homogeneous = same;
+                const int st = build_launches(n);
+                if (st) { n->failed = true; return st; }
+                BG_CUDA(cudaStreamSynchronize(n->stream));
+            }
+        }
     }
     return BG_OK;
 }
@@ -2475,6 +2493,73 @@ int bg_net_prepare(bg_net *n) {
     return st;
 }
 
+// The network's launches: the per-step list (groups, trace decay, connections
+// slot) and, where its shape allows, the persistent launch.  Called again when
+// weights written after prepare change what the launches were built from.
+static int build_launches(bg_net *n) {
+    if (n->gexec) { cudaGraphExecDestroy(n->gexec); n->gexec = nullptr; }
+    n->step_launches.clear(); n->item_names.clear(); n->finalize_launches.clear(); n->flushes.clear();
+    n->persist = nullptr; n->refill_ring = nullptr;
+    int st = plan_cluster(n);
+    if (st) return st;
+    for (size_t gi = 0; gi < n->groups.size(); ++gi) {
+        st = n->precision == 64 ? build_group<double>(n, (int)gi) : build_group<float>(n, (int)gi);
+        if (st) return st;
+    }
+    const size_t nhead = n->step_launches.size();
+    std::vector<size_t> mon_launch;
+    for (size_t si = 0; si < n->stdps.size(); ++si) { st = build_decay(n, (int)si); if (st) return st; }
+    for (const Item &it : n->items) {
+        switch (it.kind) {
+        case IT_CONN: st = n->precision == 64 ? build_conn<double>(n, it.id) : build_conn<float>(n, it.id); break;
+        case IT_SPIKEMON: mon_launch.push_back(n->step_launches.size()); st = build_spikemon(n, it.id); break;
+        // STDP keeps FP64 traces and weight arithmetic on both paths (the
+        // FP32 path moves the neuron state and the propagation to FP32)
+        case IT_STDP_PRE: st = build_stdp_pre(n, it.id); break;
+        case IT_STDP_POST: st = build_stdp_post(n, it.id); break;
+        }
+        if (st) return st;
+    }
+    // the 'synapses' slot: after the connections, before the resets
+    // (DelayConnection rows and resets of this step run in the next step's
+    // head kernel, so a target variable fed by both is refused at prepare)
+    // consecutive event-path objects with disjoint targets share their launches
+    for (size_t yi = 0; yi < n->syns.size();) {
+        if (!n->syns[yi].events || n->syns[yi].coded) { st = build_syn(n, (int)yi); if (st) return st; ++yi; continue; }
+        std::vector<int> grp{(int)yi};
+        size_t yj = yi + 1;
+        while (yj < n->syns.size() && (int)grp.size() < bg::kSynEvMerge && n->syns[yj].events && !n->syns[yj].coded) {
+            bool ok = true;
+            for (int k : grp) ok = ok && syn_disjoint(n->syns[k], n->syns[yj]);
+            if (!ok) break;
+            grp.push_back((int)yj++);
+        }
+        st = build_syn_events(n, grp);
+        if (st) return st;
+        yi = yj;
+    }
+    if (n->step_launches.empty()) return fail(BG_EINVAL, "empty network");
+    {
+        // SpikeMonitors move to right after the group kernels (they read
+        // nothing but the spike history, which only the group kernels write)
+        std::vector<Launch> L;
+        std::vector<std::string> names;
+        std::vector<char> is_mon(n->step_launches.size(), 0);
+        for (size_t i : mon_launch) is_mon[i] = 1;
+        for (size_t i = 0; i < nhead; ++i) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
+        for (size_t i : mon_launch) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
+        for (size_t i = nhead; i < n->step_launches.size(); ++i)
+            if (!is_mon[i]) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
+        n->step_launches.swap(L);
+        n->item_names.swap(names);
+        n->side0 = nhead;
+        n->side1 = nhead + mon_launch.size();
+    }
+    if (n->allow_persist) st = n->precision == 64 ? build_persist<double>(n) : build_persist<float>(n);
+    if (!st && n->allow_persist && !n->persist) st = build_syn_persist(n);
+    return st;
+}
+
 static int prepare_impl(bg_net *n) {
     if (!n) return fail(BG_EINVAL, "net");
     if (n->prepared) return BG_OK;
@@ -2759,64 +2844,7 @@ static int prepare_impl(bg_net *n) {
     BG_CUDA(cudaStreamSynchronize(n->stream));
     int st = reset_dynamic(n);
     if (st) return st;
-    // ---- per-step launch list: groups, trace decay, connections slot
-    st = plan_cluster(n);
-    if (st) return st;
-    for (size_t gi = 0; gi < n->groups.size(); ++gi) {
-        st = n->precision == 64 ? build_group<double>(n, (int)gi) : build_group<float>(n, (int)gi);
-        if (st) return st;
-    }
-    const size_t nhead = n->step_launches.size();
-    std::vector<size_t> mon_launch;
-    for (size_t si = 0; si < n->stdps.size(); ++si) { st = build_decay(n, (int)si); if (st) return st; }
-    for (const Item &it : n->items) {
-        switch (it.kind) {
-        case IT_CONN: st = n->precision == 64 ? build_conn<double>(n, it.id) : build_conn<float>(n, it.id); break;
-        case IT_SPIKEMON: mon_launch.push_back(n->step_launches.size()); st = build_spikemon(n, it.id); break;
-        // STDP keeps FP64 traces and weight arithmetic on both paths (the
-        // FP32 path moves the neuron state and the propagation to FP32)
-        case IT_STDP_PRE: st = build_stdp_pre(n, it.id); break;
-        case IT_STDP_POST: st = build_stdp_post(n, it.id); break;
-        }
-        if (st) return st;
-    }
-    // the 'synapses' slot: after the connections, before the resets
-    // (DelayConnection rows and resets of this step run in the next step's
-    // head kernel, so a target variable fed by both is refused at prepare)
-    // consecutive event-path objects with disjoint targets share their launches
-    for (size_t yi = 0; yi < n->syns.size();) {
-        if (!n->syns[yi].events || n->syns[yi].coded) { st = build_syn(n, (int)yi); if (st) return st; ++yi; continue; }
-        std::vector<int> grp{(int)yi};
-        size_t yj = yi + 1;
-        while (yj < n->syns.size() && (int)grp.size() < bg::kSynEvMerge && n->syns[yj].events && !n->syns[yj].coded) {
-            bool ok = true;
-            for (int k : grp) ok = ok && syn_disjoint(n->syns[k], n->syns[yj]);
-            if (!ok) break;
-            grp.push_back((int)yj++);
-        }
-        st = build_syn_events(n, grp);
-        if (st) return st;
-        yi = yj;
-    }
-    if (n->step_launches.empty()) return fail(BG_EINVAL, "empty network");
-    {
-        // SpikeMonitors move to right after the group kernels (they read
-        // nothing but the spike history, which only the group kernels write)
-        std::vector<Launch> L;
-        std::vector<std::string> names;
-        std::vector<char> is_mon(n->step_launches.size(), 0);
-        for (size_t i : mon_launch) is_mon[i] = 1;
-        for (size_t i = 0; i < nhead; ++i) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
-        for (size_t i : mon_launch) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
-        for (size_t i = nhead; i < n->step_launches.size(); ++i)
-            if (!is_mon[i]) { L.push_back(n->step_launches[i]); names.push_back(n->item_names[i]); }
-        n->step_launches.swap(L);
-        n->item_names.swap(names);
-        n->side0 = nhead;
-        n->side1 = nhead + mon_launch.size();
-    }
-    if (n->allow_persist) st = n->precision == 64 ? build_persist<double>(n) : build_persist<float>(n);
-    if (!st && n->allow_persist && !n->persist) st = build_syn_persist(n);
+    st = build_launches(n);
     if (st) return st;
     BG_CUDA(cudaStreamSynchronize(n->stream));
     n->prepared = true;
@@ -3934,8 +3962,12 @@ int bg_batch_free(bg_batch *b) {
 int bg_batch_run(bg_batch *b, const int64_t *nsteps, const int64_t *cs0) {
     if (!b || !nsteps || !cs0) return fail(BG_EINVAL, "bg_batch_run");
     BG_CUDA(cudaSetDevice(b->device));
-    for (bg_net *n : b->nets) {
+    for (size_t i = 0; i < b->nets.size(); ++i) {
+        bg_net *n = b->nets[i];
         if (n->failed) return fail(BG_ESTATE, "a network of the batch stopped after a device error");
+        // (weights written since the batch was made may no longer be shared)
+        const std::string why = batch_refusal(n);
+        if (!why.empty()) return fail(BG_ENOSYS, "network " + std::to_string(i) + ": " + why);
         BG_CUDA(cudaStreamSynchronize(n->stream));
     }
     return b->precision == 64 ? batch_run_impl<double>(b, nsteps, cs0) : batch_run_impl<float>(b, nsteps, cs0);
