@@ -216,6 +216,11 @@ struct HConn {
     int64_t *dColptr = nullptr, *dColk = nullptr; int32_t *dColsrc = nullptr;
     int64_t wcount() const { return dense ? sn * tn : nnz; }
 };
+// The one weight of a homogeneous connection (0 where it has no synapses).
+static double shared_weight(const HConn &c) {
+    if (c.w.empty()) return 0.0;
+    return c.w_bits == 64 ? *(const double *)c.w.data() : (double)*(const float *)c.w.data();
+}
 struct HStdp {
     int cid; double a_pre, c_pre, a_post, c_post, Ap, Am, wmin, wmax; int inter; int pre_delay, post_delay;
     double *dApre = nullptr, *dApost = nullptr; bool fused = false;
@@ -1386,7 +1391,7 @@ int build_cluster(bg_net *net, const bg::PersistArgs<T> &a, bool diag) {
         q.direct = persist_direct(h); q.md = p.rows[c]; q.emd = h.md;
         q.tablen = h.tablen; q.table = (const T *)h.dTable;
         q.off_ring = p.off_ring[c]; q.off_rows = p.off_rows[c]; q.off_syn = p.off_syn[c]; q.off_tab = p.off_tab[c];
-        q.w = (T)(h.w_bits == 64 ? *(const double *)h.w.data() : (double)*(const float *)h.w.data());
+        q.w = (T)shared_weight(h);
         q.rowptr = h.dRow; q.packed = a.push[c].packed; q.cring = h.dCRing; q.tnp = h.tnp;
         q.events = a.push[c].events;
         if (!q.packed && h.nnz > 0) return fail(BG_ESTATE, "cluster kernel: synapses not packed");
@@ -1481,8 +1486,7 @@ int build_persist(bg_net *net) {
                 return fail(BG_ENOMEM, "count ring");
             BG_CUDA(cudaMemsetAsync(c.dDirRing, 0, (size_t)c.dir_md * c.tnp * 2, net->stream));
         }
-        const double w0 = c.w_bits == 64 ? *(const double *)c.w.data() : (double)*(const float *)c.w.data();
-        const T tab[2] = {T(0), (T)w0};
+        const T tab[2] = {T(0), (T)shared_weight(c)};
         st = upload(net, c.dDirTable, tab, sizeof(tab));
         if (st) return st;
         BG_CUDA(cudaStreamSynchronize(net->stream));
@@ -2666,7 +2670,7 @@ static int prepare_impl(bg_net *n) {
                 c.tnp = (c.tn + 1) & ~1ll;
                 if (n->alloc(&c.dCRing, (size_t)c.md * c.tnp * 2) != cudaSuccess) return fail(BG_ENOMEM, "count ring");
                 if (n->alloc(&c.dTable, (size_t)(kmax + 1) * ts) != cudaSuccess) return fail(BG_ENOMEM, "count table");
-                const double w0 = c.w_bits == 64 ? *(const double *)c.w.data() : (double)*(const float *)c.w.data();
+                const double w0 = shared_weight(c);
                 if (n->precision == 64) {
                     std::vector<double> tab(kmax + 1, 0.0);
                     for (int64_t k = 1; k <= kmax; ++k) tab[k] = tab[k - 1] + w0;
@@ -3621,8 +3625,7 @@ void batch_image(bg_batch *b, const std::vector<int64_t> &nsteps, int dry, std::
             q.md = q.direct ? 2 : hc.md;           // a Connection's row of step t (parity), pushed and delivered
             q.tnp = (int32_t)((hc.tn + 1) & ~1ll);
             q.smem_ring = b->smem_ring[c][i]; q.smem_rows = b->smem_rows[c][i];
-            const double w0 = hc.w_bits == 64 ? *(const double *)hc.w.data() : (double)*(const float *)hc.w.data();
-            q.w = (T)w0;
+            q.w = (T)shared_weight(hc);
             q.rowptr = hc.dRow; q.packed = b->packed[c][i];
             q.ring = q.direct ? nullptr : hc.dCRing;
         }
