@@ -84,6 +84,8 @@ ENGINE_ONLY = {
     "group_use_buffer": [_vp, _i32, _i32],
     "group_padded_size": [_vp, _i32, _P(_i64)],
     "net_debug_hold_arrival": [_vp, _i32],
+    "net_debug_refuse_cluster": [_vp, ct.c_int],
+    "net_cluster_shape": [_vp, _P(_i32), _P(_i32)],
     "net_set_check_finite": [_vp, ct.c_int],
     "fit_compile_check": [ct.c_int, _vp, _dbl, ct.c_int, ct.c_int, ct.c_char_p, _i64],
     "fit_create": [_P(_vp), ct.c_int, ct.c_int, _vp, _dbl, ct.c_int, ct.c_int],
@@ -255,6 +257,10 @@ class Runtime(object):
         """Test hook of the bounded waits: persistent block `block` never
         publishes its step arrivals (set before prepare)."""
         self.t.check(self.t.net_debug_hold_arrival(self.h, int(block)), "net_debug_hold_arrival")
+
+    def debug_refuse_cluster(self):
+        """Test hook: prepare as on a device that places no thread-block cluster."""
+        self.t.check(self.t.net_debug_refuse_cluster(self.h, 1), "net_debug_refuse_cluster")
 
     def close(self):
         if self.h:
@@ -542,6 +548,10 @@ class Runtime(object):
             th = _i32()
             self._c(self.t.net_persistent_threads(self.h, ct.byref(th)), "net_persistent_threads")
             out["persistent_threads"] = th.value
+        if hasattr(self.t, "net_cluster_shape"):
+            blocks, npt = _i32(), _i32()
+            self._c(self.t.net_cluster_shape(self.h, ct.byref(blocks), ct.byref(npt)), "net_cluster_shape")
+            out["cluster_blocks"], out["cluster_npt"] = blocks.value, npt.value
         return out
 
 

@@ -316,6 +316,7 @@ struct bg_net {
     struct ClusterPlan {
         int npt = 0, blocks = 0, rows[2] = {0, 0}, off_ring[2] = {0, 0}, off_rows[2] = {0, 0}, off_syn[2] = {-1, -1}, off_tab[2] = {-1, -1},
             off_rec = 0;
+        int pat = 0;                   // cluster_body's PAT
         size_t smem = 0;
     } cluster;
     unsigned int *dArrived = nullptr;
@@ -327,6 +328,7 @@ struct bg_net {
     int64_t launches = 0; double last_ms = 0;
     unsigned int spin_limit = BG_SPIN_LIMIT;   // polls of a bounded inter-block wait
     int hold_block = -1;                // test hook: a persistent block that never arrives
+    bool refuse_cluster = false;        // test hook: as on a device that places no cluster
     int check_finite = 0;               // check the states for NaN/inf after every run
     bool failed = false;                // a device error stopped the network
     int syn_events_forced = 0;          // Synapses: event path whatever the size (tests)
@@ -1349,6 +1351,43 @@ int plan_cluster(bg_net *net) {
     return BG_OK;
 }
 
+// The planned network's connections in delivery order: the zero-delay
+// Connections, then the DelayConnections.
+std::vector<int> cluster_order(const bg_net *net) {
+    std::vector<int> order;
+    for (size_t c = 0; c < net->conns.size(); ++c)
+        if (persist_direct(net->conns[c])) order.push_back((int)c);
+    for (int c : net->groups[0].delivs) order.push_back(c);
+    // onto different variables the order does not matter: ascending variables
+    if (order.size() == 2 && net->conns[order[0]].var > net->conns[order[1]].var) std::swap(order[0], order[1]);
+    return order;
+}
+
+// What is left of the plan: the constant form (PAT) that the delivered
+// variables, threshold and reset have, and, for a generated model, its kernel
+// and whether the device runs the cluster.  Where it does not, or the kernel
+// does not compile, the group takes its stepped launches; so this comes before
+// those are built.
+template <typename T>
+void settle_cluster(bg_net *net) {
+    bg_net::ClusterPlan &p = net->cluster;
+    if (!p.npt) return;
+    HGroup &g = net->groups[0];
+    const std::vector<int> order = cluster_order(net);
+    bool one = true, zero = true, up = true;
+    for (size_t d = 0; d < order.size(); ++d) {
+        const int v = net->conns[order[d]].var;
+        up = up && v == (int)d + 1; one = one && v == 1; zero = zero && v == 0;
+    }
+    const bool thr = !g.gen_threshold.empty() || (g.thr_kind == BG_THR_CONST && g.thr_var == 0);
+    const bool rst = !g.gen_reset.empty() || (g.reset_kind == BG_RESET_CONST && g.reset_var == 0);
+    p.pat = !thr || !rst ? 0 : one ? 2 : up ? 1 : zero ? 3 : 0;
+    if (!g.generated()) return;
+    if (net->refuse_cluster || compile_generated_cluster<T>(g, p.npt, p.blocks > 1, p.pat) != BG_OK ||
+        !bg_cluster_fits((const void *)g.gen_ckernel, g.gen_ckernel, p.blocks, p.smem))
+        p.npt = 0;
+}
+
 // The cluster kernel's launch for the planned shape, from the persistent
 // kernel's arguments.
 template <typename T>
@@ -1362,27 +1401,8 @@ int build_cluster(bg_net *net, const bg::PersistArgs<T> &a, bool diag) {
     k.linear = g.linear; k.dt = net->dt;
     k.thr_kind = a.thr_kind; k.thr_var = a.thr_var; k.thr_var2 = a.thr_var2; k.thr_val = a.thr_val;
     k.reset_kind = a.reset_kind; k.reset_var = a.reset_var; k.reset_var2 = a.reset_var2; k.reset_val = a.reset_val;
-    // in delivery order: the zero-delay Connections, then the DelayConnections
-    std::vector<int> order;
-    for (size_t c = 0; c < net->conns.size(); ++c)
-        if (persist_direct(net->conns[c])) order.push_back((int)c);
-    for (int c : g.delivs) order.push_back(c);
-    // onto different variables the order does not matter: ascending variables
-    if (order.size() == 2 && net->conns[order[0]].var > net->conns[order[1]].var) std::swap(order[0], order[1]);
+    const std::vector<int> order = cluster_order(net);
     k.nconn = (int)order.size();
-    // the constant form that the delivered variables, threshold and reset have
-    int pat = 0;
-    {
-        bool one = true, zero = true, up = true;
-        for (int d = 0; d < k.nconn; ++d) {
-            const int v = net->conns[order[d]].var;
-            up = up && v == d + 1; one = one && v == 1; zero = zero && v == 0;
-        }
-        pat = one ? 2 : up ? 1 : zero ? 3 : 0;
-        const bool thr = !g.gen_threshold.empty() || (a.thr_kind == BG_THR_CONST && a.thr_var == 0);
-        const bool rst = !g.gen_reset.empty() || (a.reset_kind == BG_RESET_CONST && a.reset_var == 0);
-        if (!thr || !rst) pat = 0;
-    }
     for (int d = 0; d < k.nconn; ++d) {
         const int c = order[d];
         const HConn &h = net->conns[c];
@@ -1403,17 +1423,10 @@ int build_cluster(bg_net *net, const bg::PersistArgs<T> &a, bool diag) {
     k.nrec = a.nrec;
     for (int r = 0; r < a.nrec; ++r) k.rec[r] = a.rec[r];
     k.off_rec = p.off_rec;
-    const void *kern = nullptr;
-    if (g.generated()) {
-        const int st = compile_generated_cluster<T>(g, p.npt, p.blocks > 1, pat);
-        if (st) return st;
-        kern = (const void *)g.gen_ckernel;
-    } else {
-        kern = bg_cluster_kernel(sizeof(T) * 8, g.nvar, p.npt, diag, p.blocks > 1, pat);
-    }
-    if (!bg_cluster_fits(kern, g.gen_ckernel, p.blocks, p.smem)) {
-        if (!g.generated()) { net->cluster.npt = 0; return BG_OK; }
-        return fail(BG_ECUDA, "cluster kernel: no room for the cluster");
+    const void *kern = (const void *)g.gen_ckernel;          // (settle_cluster saw that it fits)
+    if (!g.generated()) {
+        kern = bg_cluster_kernel(sizeof(T) * 8, g.nvar, p.npt, diag, p.blocks > 1, p.pat);
+        if (net->refuse_cluster || !bg_cluster_fits(kern, nullptr, p.blocks, p.smem)) { net->cluster.npt = 0; return BG_OK; }
     }
     const int blocks = p.blocks;
     const size_t smem = p.smem;
@@ -2506,6 +2519,7 @@ static int build_launches(bg_net *n) {
     n->persist = nullptr; n->refill_ring = nullptr;
     int st = plan_cluster(n);
     if (st) return st;
+    if (n->precision == 64) settle_cluster<double>(n); else settle_cluster<float>(n);
     for (size_t gi = 0; gi < n->groups.size(); ++gi) {
         st = n->precision == 64 ? build_group<double>(n, (int)gi) : build_group<float>(n, (int)gi);
         if (st) return st;
@@ -3392,6 +3406,21 @@ int bg_net_debug_hold_arrival(bg_net *n, int32_t block) {
     if (!n || block < -1) return fail(BG_EINVAL, "block index");
     if (n->prepared) return fail(BG_ESTATE, "set before prepare");
     n->hold_block = block;
+    return BG_OK;
+}
+
+int bg_net_debug_refuse_cluster(bg_net *n, int refuse) {
+    if (!n) return fail(BG_EINVAL, "net");
+    if (n->prepared) return fail(BG_ESTATE, "set before prepare");
+    n->refuse_cluster = refuse != 0;
+    return BG_OK;
+}
+
+int bg_net_cluster_shape(bg_net *n, int32_t *blocks, int32_t *npt) {
+    if (!n || !blocks || !npt) return fail(BG_EINVAL, "net");
+    if (!n->prepared) { int st = bg_net_prepare(n); if (st) return st; }
+    *npt = n->persist ? n->cluster.npt : 0;
+    *blocks = *npt ? n->cluster.blocks : 0;
     return BG_OK;
 }
 

@@ -170,6 +170,8 @@ BG_API int bg_conn_add_dense(bg_net *net, int32_t src_gid, int64_t src_origin,
 BG_API int bg_conn_get_weights(bg_net *net, int32_t cid, double *out);
 /* The same weights in the connection's own type; bytes: their whole size. */
 BG_API int bg_conn_read_weights(bg_net *net, int32_t cid, void *out, int64_t bytes);
+/* New weights, before or after bg_net_prepare (a shared-weight delayed
+ * connection takes equal ones only after it, else BG_ENOSYS). */
 BG_API int bg_conn_set_weights(bg_net *net, int32_t cid, const double *in);
 
 /* ExponentialSTDP / STDP (stdp.py:181-539) on a non-delayed connection.
@@ -310,6 +312,9 @@ BG_API int bg_net_set_persistent(bg_net *net, int enable);
 /* Threads per block of the persistent kernel the prepared network runs
  * with, or 0 when it runs the general per-step launches. */
 BG_API int bg_net_persistent_threads(bg_net *net, int32_t *threads);
+/* Blocks and neurons per thread of the cluster kernel the prepared network
+ * runs in, or 0 and 0 when it runs in another one. */
+BG_API int bg_net_cluster_shape(bg_net *net, int32_t *blocks, int32_t *npt);
 /* ---- borrowed device buffers --------------------------------------------
  * Device memory the caller owns (a torch tensor, another library's buffer)
  * registered with the network; the library never frees it.  bytes >= what
@@ -365,6 +370,9 @@ BG_API int bg_net_set_spin_limit(bg_net *net, int64_t polls);
  * never publishes its step arrivals, so the other blocks' waits run out
  * (-1, the default: off).  Set before bg_net_prepare. */
 BG_API int bg_net_debug_hold_arrival(bg_net *net, int32_t block);
+/* Test hook: with refuse = 1 the network is prepared as on a device that
+ * places no thread-block cluster.  Set before bg_net_prepare. */
+BG_API int bg_net_debug_refuse_cluster(bg_net *net, int refuse);
 /* With enable = 1, every bg_net_run ends with a scan of all state
  * variables; a NaN or infinity returns BG_ENUMERIC naming the group,
  * variable and neuron, and the network refuses further runs. */
