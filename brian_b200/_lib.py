@@ -85,6 +85,7 @@ ENGINE_ONLY = {
     "group_padded_size": [_vp, _i32, _P(_i64)],
     "net_debug_hold_arrival": [_vp, _i32],
     "net_debug_refuse_cluster": [_vp, ct.c_int],
+    "net_debug_hold_cluster": [_vp, _i32],
     "net_cluster_shape": [_vp, _P(_i32), _P(_i32)],
     "net_set_check_finite": [_vp, ct.c_int],
     "fit_compile_check": [ct.c_int, _vp, _dbl, ct.c_int, ct.c_int, ct.c_char_p, _i64],
@@ -257,6 +258,10 @@ class Runtime(object):
         """Test hook of the bounded waits: persistent block `block` never
         publishes its step arrivals (set before prepare)."""
         self.t.check(self.t.net_debug_hold_arrival(self.h, int(block)), "net_debug_hold_arrival")
+
+    def debug_hold_cluster(self, block):
+        """The same for block `block` of the cluster kernel."""
+        self.t.check(self.t.net_debug_hold_cluster(self.h, int(block)), "net_debug_hold_cluster")
 
     def debug_refuse_cluster(self):
         """Test hook: prepare as on a device that places no thread-block cluster."""

@@ -34,9 +34,14 @@
 // step t'-1 (split: t'-2), so a row delivered at step t may be pushed to from
 // step t+3 (split: t+4) on: a zero-delay ring has 3 rows, a delay ring at
 // least dmax + 4.  A step's mbarrier (t mod 4) is used again four steps
-// later, when every block has long passed the wait on it.  Every wait is
-// bounded (BG_DERR_TIMEOUT); a block that gives up leaves the loop with all
-// its warps and waits in the hardware cluster barrier at the end.
+// later, when every block has long passed the wait on it.
+//
+// Every wait is bounded, by polls and by time (a poll may suspend its warp for
+// as long as the hardware sees fit).  A thread that gives up raises
+// BG_DERR_TIMEOUT and has no more spikes, its block leaves the loop at the next
+// block barrier, and the others follow as their waits run out.  Pushes of
+// theirs may still be on their way then, so no block may leave the kernel on
+// the cluster barrier alone: cluster_land waits until all of them have landed.
 //
 // What bounds it: the step's chain and the instructions of its 4 to 8 warps a
 // scheduler.  Us per step, FP64, in-degree 80 without delays (n = 1000 / 4000
@@ -80,7 +85,8 @@ template <typename T> struct ClusterArgs {
     int split;                                 // every delay >= 1: a step waits for the step before it
     unsigned long long *spikes;
     int nsteps;
-    unsigned int spin_limit;                   // polls of a wait before it gives up
+    unsigned int spin_limit;                   // polls, and microseconds, of a wait before it gives up
+    int hold_block;                            // test hook: this block never publishes its arrivals (-1: none)
     uint32_t *mon_words; int mon_stride;       // spike words per step of the launch, or null
     int nrec; RecDev rec[kMaxRec]; int off_rec;   // StateMonitors; first entry of each neuron [nrec][BN + 1]
 };
@@ -102,14 +108,58 @@ __device__ __forceinline__ void cluster_push(uint32_t addr, uint32_t v, uint32_t
 __device__ __forceinline__ void cluster_arrive_tx(uint32_t mbar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" :: "r"(mbar), "r"(bytes) : "memory");
 }
+// the bytes without the arrival
+__device__ __forceinline__ void cluster_expect_tx(uint32_t mbar, uint32_t bytes) {
+    asm volatile("mbarrier.expect_tx.relaxed.cluster.shared::cluster.b64 [%0], %1;" :: "r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool cluster_try(uint32_t mbar, uint32_t parity) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+// A thread's wait for a phase of an mbarrier; false when it gave up.  (The time
+// is looked at every 64 polls of a loop that is not unrolled: a timed loop behind
+// a few plain polls cost 4 to 6 % of a step.)
 __device__ __forceinline__ bool cluster_wait(uint32_t mbar, uint32_t parity, unsigned int limit) {
+    unsigned long long until = 0;
+#pragma unroll 1
     for (unsigned int i = 0; i <= limit; ++i) {
-        uint32_t done;
-        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                     " selp.u32 %0, 1, 0, p;\n}" : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
-        if (done) return true;
+        if (cluster_try(mbar, parity)) return true;
+        if ((i & 63) == 63) {
+            const unsigned long long t = global_ns();
+            if (!until) until = t + 1000ull * limit;
+            else if (t > until) return false;
+        }
     }
     return false;
+}
+
+// After a wait has run out somewhere in the cluster, and a cluster barrier:
+// called by one warp of every block, it returns when all pushes into the block
+// have landed.  `count`: arrivals each block sent every block, by mbarrier.  Each
+// push's bytes were announced, so a phase completes when its bytes have landed and
+// its arrivals are there; the missing arrivals of the last, incomplete phase are
+// made up here.
+__device__ __forceinline__ void cluster_land(uint32_t mb0, uint32_t count, int blocks, int lane, unsigned int limit) {
+    for (int i = 0; i < 4; ++i) {
+        uint32_t sent = 0;
+        if (lane < blocks)
+            asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(sent) : "r"(cluster_addr(count + 4 * i, lane)) : "memory");
+        sent = __reduce_add_sync(0xffffffffu, sent);
+        const uint32_t phases = (sent + blocks - 1) / blocks;
+        if (lane == 0)
+            for (uint32_t k = sent; k < phases * blocks; ++k)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mb0 + 8 * i) : "memory");
+        __syncwarp();
+        if (phases) cluster_wait(mb0 + 8 * i, (phases - 1) & 1, limit);
+        __syncwarp();
+    }
 }
 
 // 1 << var where the compiler cannot see that one bit is set: a chain of tests
@@ -145,6 +195,8 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
     extern __shared__ __align__(16) unsigned char csm[];
     __shared__ __align__(8) unsigned long long mbars[4];     // arrivals and bytes of the steps t mod 4
     __shared__ uint32_t sent[2][kClusterMaxBlocks];          // pushes of this block to each block, steps t mod 2
+    __shared__ uint32_t count[4];                            // arrivals sent to every block, by mbarrier
+    __shared__ uint32_t failed;                              // a wait has run out in some block
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
     const int blocks = gridDim.x;                  // the grid is one cluster: block rank = block index
     const int base = blockIdx.x * BN;
@@ -161,6 +213,7 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         for (int k = tid; k < 2 * kClusterMaxBlocks; k += nth) sent[k / kClusterMaxBlocks][k % kClusterMaxBlocks] = 0;
+        if (tid == 0) failed = 0;
     }
     // ---- staging: rings (row k: due at step t0 + k), row starts (relative to
     // the block's first), synapses, tables
@@ -224,17 +277,32 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
 
     if (MULTI && warp == TH / 32) {
         // ---- the 17th warp: one arrival per block and step
-        for (int st = 0; st < a.nsteps; ++st) {
-            if (__syncthreads_or(0)) break;
+        const bool held = (int)blockIdx.x == a.hold_block;
+        int st = 0;
+        uint32_t extra = 0;
+        for (; st < a.nsteps; ++st) {
+            const bool stop = __syncthreads_or(0);
+            const uint32_t n = lane < blocks ? sent[st & 1][lane] : 0;
+            // (a block that stops has pushed only where a thread's last wait did not run out)
+            if (stop && !__any_sync(0xffffffffu, n != 0)) break;
             if (lane < blocks) {
-                const uint32_t bytes = 4u * sent[st & 1][lane];
                 sent[st & 1][lane] = 0;            // next used at step st + 2, past the barrier of step st + 1
-                cluster_arrive_tx(cluster_addr(mb0 + 8 * (st & 3), lane), bytes);
+                const uint32_t mbar = cluster_addr(mb0 + 8 * (st & 3), lane);
+                if (held) cluster_expect_tx(mbar, 4u * n);
+                else cluster_arrive_tx(mbar, 4u * n);
             }
             __syncwarp();
             asm volatile("fence.acq_rel.cluster;" ::: "memory");
+            if (stop) { extra = 1; break; }
         }
+        if (lane < 4) count[lane] = held ? 0 : (uint32_t)(st + extra + 3 - lane) / 4;     // steps lane, lane + 4, ...
+        __syncwarp();
         cluster_sync();
+        if (failed) {                              // uniform over the cluster
+            cluster_land(mb0, (uint32_t)__cvta_generic_to_shared(count), blocks, lane, a.spin_limit);
+            __syncwarp();
+            cluster_sync();                        // every block's counts are read
+        }
         return;
     }
 
@@ -268,6 +336,7 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
     for (int u = 0; u < NPT; ++u)
         if (mon && lane == 0 && ((base + u * TH + warp * 32) >> 5) < a.mon_stride) monmask |= 1u << u;
     bool gave_up = false;
+    int live = nvalid;                             // neurons that may spike: none once the thread has given up
     int st = 0;
     for (; st < a.nsteps; ++st) {
         const double tm = __dmul_rn((double)(cs0 + st), a.dt);   // time of the step (generated models)
@@ -310,7 +379,7 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
 #pragma unroll
         for (int u = 0; u < NPT; ++u) {
             const int wb = u * TH + warp * 32;     // neuron of bit 0 within the block
-            spk[u] = spk[u] && wb + lane < nvalid;
+            spk[u] = spk[u] && wb + lane < live;
             const uint32_t ball = __ballot_sync(0xffffffffu, spk[u]);
             if ((monmask >> u) & 1u) mon[u * (TH / 32)] = ball;
             if (!ball) continue;                   // warp-uniform
@@ -353,6 +422,7 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
             if (__syncthreads_or(gave_up)) break;  // uniform over the block
             if (!a.split) gave_up = !cluster_wait(mbar, (st >> 2) & 1, a.spin_limit);
             else if (st > 0) gave_up = !cluster_wait(mb0 + 8 * ((st - 1) & 3), ((st - 1) >> 2) & 1, a.spin_limit);
+            if (gave_up) live = 0;
         } else {
             __syncthreads();
         }
@@ -456,9 +526,15 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
         // leaves while another may still send to it
         if (a.split && !gave_up && st == a.nsteps && st > 0)
             gave_up = !cluster_wait(mb0 + 8 * ((st - 1) & 3), ((st - 1) >> 2) & 1, a.spin_limit);
-        if (gave_up) bg_raise(a.ctl, BG_DERR_TIMEOUT, t0 + st);
+        if (__any_sync(0xffffffffu, gave_up)) {
+            bg_raise(a.ctl, BG_DERR_TIMEOUT, t0 + st);
+            if (lane < blocks)
+                asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;"
+                             :: "r"(cluster_addr((uint32_t)__cvta_generic_to_shared(&failed), lane)), "r"(1u) : "memory");
+        }
         __syncwarp();
         cluster_sync();
+        if (failed) cluster_sync();                // (cluster_land, by the 17th warp)
     } else {
         __syncthreads();
     }

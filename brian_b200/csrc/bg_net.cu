@@ -329,6 +329,7 @@ struct bg_net {
     unsigned int spin_limit = BG_SPIN_LIMIT;   // polls of a bounded inter-block wait
     int hold_block = -1;                // test hook: a persistent block that never arrives
     bool refuse_cluster = false;        // test hook: as on a device that places no cluster
+    int hold_cluster = -1;              // test hook: a block of the cluster kernel that never arrives
     int check_finite = 0;               // check the states for NaN/inf after every run
     bool failed = false;                // a device error stopped the network
     int syn_events_forced = 0;          // Synapses: event path whatever the size (tests)
@@ -1417,6 +1418,7 @@ int build_cluster(bg_net *net, const bg::PersistArgs<T> &a, bool diag) {
         if (!q.packed && h.nnz > 0) return fail(BG_ESTATE, "cluster kernel: synapses not packed");
     }
     k.spin_limit = a.spin_limit;
+    k.hold_block = net->hold_cluster;
     k.split = a.lag == 2;
     k.spikes = a.spikes;
     k.mon_words = a.mon_words; k.mon_stride = (int)a.mon_stride;
@@ -3413,6 +3415,13 @@ int bg_net_debug_refuse_cluster(bg_net *n, int refuse) {
     if (!n) return fail(BG_EINVAL, "net");
     if (n->prepared) return fail(BG_ESTATE, "set before prepare");
     n->refuse_cluster = refuse != 0;
+    return BG_OK;
+}
+
+int bg_net_debug_hold_cluster(bg_net *n, int32_t block) {
+    if (!n || block < -1) return fail(BG_EINVAL, "block index");
+    if (n->prepared) return fail(BG_ESTATE, "set before prepare");
+    n->hold_cluster = block;
     return BG_OK;
 }
 

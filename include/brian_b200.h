@@ -362,7 +362,8 @@ BG_API int bg_net_load(bg_net *net, const char *path);
 /* ---- failure detection (no counterpart in the reference, where a stalled
  * or diverging simulation just runs on) -------------------------------------
  * Polls of the persistent kernel's bounded inter-block wait before it gives
- * up (default 2^22, a few seconds): every block then leaves its step loop,
+ * up (default 2^22, a few seconds; in the cluster kernel, whose polls may
+ * suspend, also microseconds): every block then leaves its step loop,
  * bg_net_run returns BG_ETIMEOUT with no kernel left running, and the
  * network refuses further runs (BG_ESTATE).  Set before bg_net_prepare. */
 BG_API int bg_net_set_spin_limit(bg_net *net, int64_t polls);
@@ -370,6 +371,8 @@ BG_API int bg_net_set_spin_limit(bg_net *net, int64_t polls);
  * never publishes its step arrivals, so the other blocks' waits run out
  * (-1, the default: off).  Set before bg_net_prepare. */
 BG_API int bg_net_debug_hold_arrival(bg_net *net, int32_t block);
+/* The same for block `block` of the cluster kernel, where it has several. */
+BG_API int bg_net_debug_hold_cluster(bg_net *net, int32_t block);
 /* Test hook: with refuse = 1 the network is prepared as on a device that
  * places no thread-block cluster.  Set before bg_net_prepare. */
 BG_API int bg_net_debug_refuse_cluster(bg_net *net, int refuse);
