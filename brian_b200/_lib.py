@@ -85,6 +85,8 @@ ENGINE_ONLY = {
     "group_padded_size": [_vp, _i32, _P(_i64)],
     "net_debug_hold_arrival": [_vp, _i32],
     "net_debug_refuse_cluster": [_vp, ct.c_int],
+    "net_debug_device_limit": [_vp, _i64],
+    "net_device_bytes": [_vp, _P(_i64)],
     "net_debug_hold_cluster": [_vp, _i32],
     "net_cluster_shape": [_vp, _P(_i32), _P(_i32)],
     "net_set_check_finite": [_vp, ct.c_int],
@@ -262,6 +264,10 @@ class Runtime(object):
     def debug_hold_cluster(self, block):
         """The same for block `block` of the cluster kernel."""
         self.t.check(self.t.net_debug_hold_cluster(self.h, int(block)), "net_debug_hold_cluster")
+
+    def debug_device_limit(self, nbytes):
+        """Test hook: allocations past nbytes of device memory in all fail."""
+        self.t.check(self.t.net_debug_device_limit(self.h, int(nbytes)), "net_debug_device_limit")
 
     def debug_refuse_cluster(self):
         """Test hook: prepare as on a device that places no thread-block cluster."""
@@ -557,6 +563,10 @@ class Runtime(object):
             blocks, npt = _i32(), _i32()
             self._c(self.t.net_cluster_shape(self.h, ct.byref(blocks), ct.byref(npt)), "net_cluster_shape")
             out["cluster_blocks"], out["cluster_npt"] = blocks.value, npt.value
+        if hasattr(self.t, "net_device_bytes"):
+            nbytes = _i64()
+            self._c(self.t.net_device_bytes(self.h, ct.byref(nbytes)), "net_device_bytes")
+            out["device_bytes"] = nbytes.value
         return out
 
 

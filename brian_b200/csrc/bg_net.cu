@@ -322,7 +322,7 @@ struct bg_net {
     unsigned int *dArrived = nullptr;
     // Synapses persistent kernel: the ring of bins, to be filled again from
     // the history before the next launch when stale
-    int *dRingCnt = nullptr; bg::SynRec *dRingEv = nullptr; size_t ring_bins = 0;
+    int *dRingCnt = nullptr; bg::SynRec *dRingEv = nullptr; size_t ring_bins = 0; int ring_cap = 0;
     bool syn_ring_stale = true;
     std::function<int()> refill_ring;
     int64_t launches = 0; double last_ms = 0;
@@ -334,17 +334,31 @@ struct bg_net {
     bool failed = false;                // a device error stopped the network
     int syn_events_forced = 0;          // Synapses: event path whatever the size (tests)
     bool syn_lists_stale = true;        // Synapses spike lists to rebuild from the history before the next step
-    std::vector<void *> allocs;
+    std::vector<std::pair<void *, int64_t>> allocs;
     struct Import { void *ptr; int64_t bytes; int dtype; };
     std::vector<Import> imports;        // borrowed device buffers (the caller owns and frees them)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int64_t chunk_steps = kChunkSteps;
 
+    int64_t dev_bytes = 0, dev_limit = 0;   // device memory of `allocs`; test hook: as on a device with no more than this (0: off)
     template <typename P> cudaError_t alloc(P **p, size_t bytes) {
         void *q = nullptr;
-        cudaError_t e = cudaMalloc(&q, bytes ? bytes : 16);
-        if (e == cudaSuccess) { allocs.push_back(q); *p = (P *)q; }
+        if (!bytes) bytes = 16;
+        cudaError_t e = dev_limit && dev_bytes + (int64_t)bytes > dev_limit ? cudaErrorMemoryAllocation : cudaMalloc(&q, bytes);
+        if (e == cudaSuccess) { allocs.push_back({q, (int64_t)bytes}); dev_bytes += (int64_t)bytes; *p = (P *)q; }
+        else cudaGetLastError();            // (a caller may go on without the buffer)
         return e;
+    }
+    // a buffer given back before the network is destroyed
+    template <typename P> void release(P *&p) {
+        for (size_t k = 0; p && k < allocs.size(); ++k)
+            if (allocs[k].first == (void *)p) {
+                cudaFree((void *)p);
+                dev_bytes -= allocs[k].second;
+                allocs.erase(allocs.begin() + k);
+                break;
+            }
+        p = nullptr;
     }
 };
 
@@ -1713,16 +1727,6 @@ int build_syn_persist(bg_net *net) {
     int dmax = 0;
     for (const HSyn &y : net->syns) dmax = std::max(dmax, y.dmax);
     a.ring = dmax + 2;
-    // entries a bin holds: all that are ordered in shared memory, or the power of two below that fits kSPRing
-    a.cap = bg::kSynBinCap;
-    while (a.cap > bg::kSPBn && (int64_t)a.ring * a.nbins * a.cap * (int64_t)sizeof(bg::SynRec) > bg::kSPRing) a.cap /= 2;
-    if (!net->dRingCnt) {
-        net->ring_bins = (size_t)a.ring * a.nbins;
-        if (net->alloc(&net->dRingCnt, net->ring_bins * 4) != cudaSuccess ||
-            net->alloc(&net->dRingEv, net->ring_bins * a.cap * sizeof(bg::SynRec)) != cudaSuccess)
-            return fail(BG_ENOMEM, "synapse event bins");
-    }
-    a.bin_cnt = net->dRingCnt; a.bin_ev = net->dRingEv;
     for (int k = 0; k < a.nobj; ++k) {
         HSyn &y = net->syns[k];
         if (!y.dRec) {
@@ -1770,6 +1774,21 @@ int build_syn_persist(bg_net *net) {
     for (int j = 0; j < g.nvar; ++j)
         for (int k = 0; k < g.nvar; ++k)
             if ((((a.anz >> (j * g.nvar + k)) & 1ull) != 0) != (j == 0 || j == k)) diag = false;
+    // entries a bin holds: all that are ordered in shared memory, or the power
+    // of two below for which the ring fits kSPRing and the device's memory (a
+    // bin that more events reach is delivered by the pull)
+    if (!net->dRingCnt) {
+        net->ring_bins = (size_t)a.ring * a.nbins;
+        net->ring_cap = bg::kSynBinCap;
+        while (net->ring_cap > bg::kSPBn && (int64_t)net->ring_bins * net->ring_cap * (int64_t)sizeof(bg::SynRec) > bg::kSPRing) net->ring_cap /= 2;
+        if (net->alloc(&net->dRingCnt, net->ring_bins * 4) != cudaSuccess) return fail(BG_ENOMEM, "synapse event bins");
+        while (net->alloc(&net->dRingEv, net->ring_bins * net->ring_cap * sizeof(bg::SynRec)) != cudaSuccess) {
+            if (net->ring_cap <= bg::kSPBn) return fail(BG_ENOMEM, "synapse event bins");
+            net->ring_cap /= 2;
+        }
+    }
+    a.cap = net->ring_cap;
+    a.bin_cnt = net->dRingCnt; a.bin_ev = net->dRingEv;
     const void *k = kern[g.nvar - 1][diag ? 1 : 0];
     unsigned int *arr = net->dArrived;
     net->persist_used = bg::kSPTh;
@@ -1861,7 +1880,7 @@ int bg_net_destroy(bg_net *n) {
         if (g.gen_lib) cudaLibraryUnload(g.gen_lib);
         if (g.gen_clib) cudaLibraryUnload(g.gen_clib);
     }
-    for (void *p : n->allocs) cudaFree(p);
+    for (auto &p : n->allocs) cudaFree(p.first);
     if (n->ev0) cudaEventDestroy(n->ev0);
     if (n->ev1) cudaEventDestroy(n->ev1);
     if (n->ev_fork) cudaEventDestroy(n->ev_fork);
@@ -2515,7 +2534,7 @@ int bg_net_prepare(bg_net *n) {
 // The network's launches: the per-step list (groups, trace decay, connections
 // slot) and, where its shape allows, the persistent launch.  Called again when
 // weights written after prepare change what the launches were built from.
-static int build_launches(bg_net *n) {
+static int build_launches_as(bg_net *n) {
     if (n->gexec) { cudaGraphExecDestroy(n->gexec); n->gexec = nullptr; }
     n->step_launches.clear(); n->item_names.clear(); n->finalize_launches.clear(); n->flushes.clear();
     n->persist = nullptr; n->refill_ring = nullptr;
@@ -2578,6 +2597,20 @@ static int build_launches(bg_net *n) {
     if (n->allow_persist) st = n->precision == 64 ? build_persist<double>(n) : build_persist<float>(n);
     if (!st && n->allow_persist && !n->persist) st = build_syn_persist(n);
     return st;
+}
+
+// Where the device has no room for what a persistent launch keeps besides the
+// network itself, its buffers are given back and the network runs stepped.
+static int build_launches(bg_net *n) {
+    const int st = build_launches_as(n);
+    if (st != BG_ENOMEM || !n->allow_persist) return st;
+    BG_CUDA(cudaStreamSynchronize(n->stream));
+    for (HConn &c : n->conns) { n->release(c.dPacked); n->release(c.dDirRing); n->release(c.dDirTable); }
+    for (HSyn &y : n->syns) n->release(y.dRec);
+    for (HStateMon &m : n->stmons) n->release(m.dBlkP);
+    n->release(n->dRingCnt); n->release(n->dRingEv); n->release(n->dMonWords); n->release(n->dMonOff); n->release(n->dArrived);
+    n->allow_persist = 0;
+    return build_launches_as(n);
 }
 
 static int prepare_impl(bg_net *n) {
@@ -2745,15 +2778,6 @@ static int prepare_impl(bg_net *n) {
                     break;
                 }
         }
-        // on a dense connection the rule's kernels share one launch and the
-        // postsynaptic updates wait (the trace records of 64 steps: 512 bytes a source)
-        s.lazy = s.fused && c.dense && c.sn > 0 && c.tn > 0 && c.sn * bg::kLazySteps * 8 <= ((int64_t)1 << 30);
-        if (s.lazy) {
-            if (n->alloc(&s.dRec, (size_t)c.sn * bg::kLazySteps * 8) != cudaSuccess ||
-                n->alloc(&s.dRowMask, (size_t)c.sn * 16) != cudaSuccess || n->alloc(&s.dColMask, (size_t)c.tn * 16) != cudaSuccess ||
-                n->alloc(&s.dLz, sizeof(bg::LazyCtl)) != cudaSuccess)
-                return fail(BG_ENOMEM, "STDP pending updates");
-        }
     }
     for (auto &m : n->smons) {
         m.cap = std::max<int64_t>(1024, m.n * (n->chunk_steps + 1));
@@ -2861,6 +2885,17 @@ static int prepare_impl(bg_net *n) {
     const size_t ncount = n->groups.size() + n->conns.size();
     if (n->alloc(&n->dCounters, std::max<size_t>(1, ncount) * 8) != cudaSuccess) return fail(BG_ENOMEM, "counters");
     BG_CUDA(cudaMemsetAsync(n->dCounters, 0, std::max<size_t>(1, ncount) * 8, n->stream));
+    for (auto &s : n->stdps) {
+        // on a dense connection the rule's kernels share one launch and the
+        // postsynaptic updates wait (the trace records of 64 steps: 512 bytes a
+        // source), where the device has the room: every step's update else
+        const HConn &c = n->conns[s.cid];
+        if (!s.fused || !c.dense || c.sn <= 0 || c.tn <= 0 || c.sn * bg::kLazySteps * 8 > ((int64_t)1 << 30)) continue;
+        s.lazy = n->alloc(&s.dRec, (size_t)c.sn * bg::kLazySteps * 8) == cudaSuccess &&
+                 n->alloc(&s.dRowMask, (size_t)c.sn * 16) == cudaSuccess && n->alloc(&s.dColMask, (size_t)c.tn * 16) == cudaSuccess &&
+                 n->alloc(&s.dLz, sizeof(bg::LazyCtl)) == cudaSuccess;
+        if (!s.lazy) { n->release(s.dRec); n->release(s.dRowMask); n->release(s.dColMask); n->release(s.dLz); }
+    }
     BG_CUDA(cudaStreamSynchronize(n->stream));
     int st = reset_dynamic(n);
     if (st) return st;
@@ -3422,6 +3457,19 @@ int bg_net_debug_hold_cluster(bg_net *n, int32_t block) {
     if (!n || block < -1) return fail(BG_EINVAL, "block index");
     if (n->prepared) return fail(BG_ESTATE, "set before prepare");
     n->hold_cluster = block;
+    return BG_OK;
+}
+
+int bg_net_debug_device_limit(bg_net *n, int64_t bytes) {
+    if (!n || bytes < 0) return fail(BG_EINVAL, "bytes");
+    if (n->prepared) return fail(BG_ESTATE, "set before prepare");
+    n->dev_limit = bytes;
+    return BG_OK;
+}
+
+int bg_net_device_bytes(bg_net *n, int64_t *bytes) {
+    if (!n || !bytes) return fail(BG_EINVAL, "net");
+    *bytes = n->dev_bytes;
     return BG_OK;
 }
 

@@ -315,6 +315,8 @@ BG_API int bg_net_persistent_threads(bg_net *net, int32_t *threads);
 /* Blocks and neurons per thread of the cluster kernel the prepared network
  * runs in, or 0 and 0 when it runs in another one. */
 BG_API int bg_net_cluster_shape(bg_net *net, int32_t *blocks, int32_t *npt);
+/* Device memory the network holds, in bytes. */
+BG_API int bg_net_device_bytes(bg_net *net, int64_t *bytes);
 /* ---- borrowed device buffers --------------------------------------------
  * Device memory the caller owns (a torch tensor, another library's buffer)
  * registered with the network; the library never frees it.  bytes >= what
@@ -373,6 +375,9 @@ BG_API int bg_net_set_spin_limit(bg_net *net, int64_t polls);
 BG_API int bg_net_debug_hold_arrival(bg_net *net, int32_t block);
 /* The same for block `block` of the cluster kernel, where it has several. */
 BG_API int bg_net_debug_hold_cluster(bg_net *net, int32_t block);
+/* Test hook: allocations past `bytes` of device memory in all fail, as on a
+ * device with no more (0, the default: off).  Set before bg_net_prepare. */
+BG_API int bg_net_debug_device_limit(bg_net *net, int64_t bytes);
 /* Test hook: with refuse = 1 the network is prepared as on a device that
  * places no thread-block cluster.  Set before bg_net_prepare. */
 BG_API int bg_net_debug_refuse_cluster(bg_net *net, int refuse);
