@@ -446,7 +446,10 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
         for (int d = 0; d < kClusterMaxConn; ++d) {
             if (d >= a.nconn) break;
             const ClusterConn<T> &q = a.conn[d];
-            // (adding no events' 0 would change the sign of a -0 only)
+            // A DelayConnection adds its row's 0 where no event is due, too: that
+            // makes +0 of a -0, which a linear update does not leave behind but a
+            // generated one may.
+            const int i0 = base + tid - q.to;
             if constexpr (PAT != 0) {
                 constexpr int NVd = NV;
                 const int k = cluster_var<PAT>(d);
@@ -469,14 +472,15 @@ __device__ __forceinline__ void cluster_body(const ClusterArgs<T> &a) {
                     const T *tab = q.off_tab >= 0 ? reinterpret_cast<const T *>(csm + q.off_tab) : q.table;
 #pragma unroll
                     for (int u = 0; u < NPT; ++u)
-                        if (cnt[d][u]) s[u][k < NVd ? k : 0] = rn<T>::add(s[u][k < NVd ? k : 0], tab[cnt[d][u]]);
+                        if (M::custom_update ? (unsigned)(i0 + u * TH) < (unsigned)q.tn : cnt[d][u] != 0)
+                            s[u][k < NVd ? k : 0] = rn<T>::add(s[u][k < NVd ? k : 0], tab[cnt[d][u]]);
                 }
             } else {
                 const T *tab = q.off_tab >= 0 ? reinterpret_cast<const T *>(csm + q.off_tab) : q.table;
 #pragma unroll
                 for (int u = 0; u < NPT; ++u) {
                     const int n = cnt[d][u];
-                    if (!n) continue;
+                    if (!n && !(M::custom_update && !q.direct && (unsigned)(i0 + u * TH) < (unsigned)q.tn)) continue;
                     T x = pick_var<T, NV>(s[u], dvar[d]);
                     if (q.direct) {
                         for (int i = 0; i < n; ++i) x = rn<T>::add(x, q.w);

@@ -77,14 +77,18 @@ __host__ __device__ __forceinline__ void bg_philox_uniform2f(uint64_t seed, uint
 
 // Exactly-rounded arithmetic without contraction, spelled out so that no
 // compiler flag can fuse a multiply into an add on the bit-exact path.
+// mul0(a, b) is 0 + a b in one operation: the product, with +0 for a product
+// that is -0 (a negative one that underflows to zero keeps its sign).
 template <typename T> struct rn;
 template <> struct rn<double> {
     static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
     static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ double mul0(double a, double b) { return __fma_rn(a, b, 0.0); }
 };
 template <> struct rn<float> {
     static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
     static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ float mul0(float a, float b) { return __fmaf_rn(a, b, 0.0f); }
 };
 
 // Per-network control block in device memory.  Kernels of one step all read

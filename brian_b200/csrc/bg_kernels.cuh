@@ -136,25 +136,24 @@ __device__ __forceinline__ T linear_row(const T *A, const T *C, uint64_t anz, ui
     return acc;
 }
 
-// x = A s (+ C) of a thread's NPT neurons, each row summed as linear_row does
-// but without its leading 0 + (which changes the sign of a -0 only and is a
-// tenth of the FP64 work of a CUBA step); the mask tests are uniform and run
-// once per thread, not per neuron.  DIAG: the host found A's nonzeros to be
-// exactly its first row and its diagonal, and C's to be at most its first
-// entry (a potential driven by decaying synaptic variables, as in CUBA), so
-// the update needs no mask tests.
+// x = A s (+ C) of a thread's NPT neurons, each row summed as linear_row does;
+// the mask tests are uniform and run once per thread, not per neuron.  DIAG:
+// the host found A's nonzeros to be exactly its first row and its diagonal, and
+// C's to be at most its first entry (a potential driven by decaying synaptic
+// variables, as in CUBA), so the update needs no mask tests, and a row's leading
+// 0 + (a tenth of the FP64 work of a CUBA step) goes into its first product.
 template <typename T, int NV, int NPT, bool DIAG>
 __device__ __forceinline__ void linear_update(const T *A, const T *C, uint64_t anz, uint32_t cnz, T (&s)[NPT][NV]) {
     T x[NPT][NV];
     if constexpr (DIAG) {
 #pragma unroll
         for (int u = 0; u < NPT; ++u) {
-            T acc = rn<T>::mul(A[0], s[u][0]);
+            T acc = rn<T>::mul0(A[0], s[u][0]);
 #pragma unroll
             for (int k = 1; k < NV; ++k) acc = rn<T>::add(acc, rn<T>::mul(A[k], s[u][k]));
             x[u][0] = acc;
 #pragma unroll
-            for (int j = 1; j < NV; ++j) x[u][j] = rn<T>::mul(A[j * NV + j], s[u][j]);
+            for (int j = 1; j < NV; ++j) x[u][j] = rn<T>::mul0(A[j * NV + j], s[u][j]);
         }
         if (cnz & 1u) {
 #pragma unroll
