@@ -818,6 +818,7 @@ struct DecayArgs {
     double *H_pre, *H_post; int hlen;     // trace histories [hlen][n], or null
     DevCtl *ctl; int last;
 };
+#ifndef __CUDACC_RTC__
 static __global__ void k_stdp_decay(const DecayArgs a) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const long long nstep = a.ctl->nstep;
@@ -835,6 +836,7 @@ static __global__ void k_stdp_decay(const DecayArgs a) {
     }
     bg_finish_step(a.ctl, a.last);
 }
+#endif
 
 // Slot of the trace record `lag` records before the last one
 // (monitor.py:1092: (current_time_index - 1 - lag) mod M, one record per
@@ -1153,6 +1155,7 @@ struct SynArgs {
     const int *use_pull;            // event path present: [step parity] 1 = the pull delivers this step
     int last;
 };
+#ifndef __CUDACC_RTC__
 static __global__ void __launch_bounds__(kSynThreads) k_syn_deliver(const SynArgs a) {
     __shared__ uint32_t mask[kSynChunk / 32];
     const long long nstep = a.ctl->nstep;
@@ -1242,6 +1245,7 @@ static __global__ void __launch_bounds__(kSynThreads) k_syn_deliver(const SynArg
     }
     bg_finish_step(a.ctl, a.last);
 }
+#endif
 
 // Synapses with code (plastic synapses, synapses.py:149-330, 400-510): per
 // synapse variables in column order, the presynaptic code run for each event
@@ -1482,6 +1486,7 @@ __device__ __forceinline__ void syn_gather_word(const SynEvArgs &a, long long ns
     }
 }
 
+#ifndef __CUDACC_RTC__
 static __global__ void __launch_bounds__(256) k_syn_gather(const __grid_constant__ SynEvGroup g) {
     const long long nstep = g.ctl->nstep;
     const int nlist = g.pair0[g.nobj] * g.nparts;
@@ -1513,10 +1518,12 @@ static __global__ void __launch_bounds__(256) k_syn_gather(const __grid_constant
     }
     bg_finish_step(g.ctl, g.last);
 }
+#endif
 
 // The spike lists of steps t-1 .. t-dmax rebuilt from the spike history
 // (before a run whose history did not come from the gather: a new or
 // reinitialised network, a loaded state); the rows' counts are zero.
+#ifndef __CUDACC_RTC__
 static __global__ void __launch_bounds__(256) k_syn_lists(const SynEvArgs a) {
     const long long nstep = a.ctl->nstep;
     const int64_t w0 = a.so >> 5, nw = ((a.so + a.sn + 31) >> 5) - w0;
@@ -1534,6 +1541,7 @@ static __global__ void __launch_bounds__(256) k_syn_lists(const SynEvArgs a) {
         }
     }
 }
+#endif
 
 constexpr int kSynBinThreads = 512;
 constexpr int kSynTPT = kSynBin / kSynBinThreads;       // targets per thread
@@ -1739,12 +1747,14 @@ __device__ __forceinline__ void syn_bins_block(const SynEvArgs &a, long long nst
     }
 }
 
+#ifndef __CUDACC_RTC__
 static __global__ void __launch_bounds__(kSynBinThreads, 4) k_syn_bins(const __grid_constant__ SynEvGroup g) {
     int k = 0;
     while (k + 1 < g.nobj && (int)blockIdx.x >= g.bin0[k + 1]) ++k;
     syn_bins_block(g.o[k], g.ctl->nstep, (int)blockIdx.x - g.bin0[k]);
     bg_finish_step(g.ctl, g.last);
 }
+#endif
 
 // SpikeMonitor (monitor.py:156-166): one block appends the step's spikes in
 // ascending order.  A pass covers kMonThreads * kMonWords history words: they
@@ -1761,6 +1771,7 @@ struct MonArgs {
 };
 constexpr int kMonThreads = 1024;
 constexpr int kMonWords = 8;
+#ifndef __CUDACC_RTC__
 static __global__ void __launch_bounds__(kMonThreads) k_spikemon(const MonArgs a) {
     __shared__ uint32_t sw[kMonThreads * kMonWords + kMonThreads * kMonWords / 32];   // one pad word per 32: no bank conflicts either way
     __shared__ int wcnt[kMonThreads / 32];
@@ -1822,5 +1833,6 @@ static __global__ void __launch_bounds__(kMonThreads) k_spikemon(const MonArgs a
     }
     bg_finish_step(a.ctl, a.last);
 }
+#endif
 
 }  // namespace bg
