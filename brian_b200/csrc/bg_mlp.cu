@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "bg_common.cuh"
+#include "bg_deviceonce.h"
 #include "bg_mlpchain.cuh"
 #include "../../include/brian_b200.h"
 
@@ -274,18 +275,37 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const EncodeTiledFn fn = [] {
         void *p = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = (EncodeTiledFn)p;
+        const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                        q == cudaDriverEntryPointSuccess;
         cudaGetLastError();
-    }
+        return ok ? (EncodeTiledFn)p : nullptr;
+    }();
     return fn;
+}
+
+// A device and its multiprocessors.
+struct Device { int id, sms; };
+Device device_of(int id) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, id) != cudaSuccess || n <= 0) n = 148;
+    return {id, n};
+}
+
+// The dynamic shared memory that a kernel may take, raised once per device
+// (the attribute belongs to the kernel on the current device `dev`; handles on
+// several devices and threads share the kernels).
+int raise_smem(int dev, const void *kernel, size_t bytes) {
+    static DeviceOnce once;
+    cudaError_t e = cudaSuccess;
+    if (!once(dev, kernel, [&] {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+            return e == cudaSuccess;
+        }))
+        return fail(BG_ECUDA, std::string("mlp: shared memory of a kernel: ") + cudaGetErrorString(e));
+    return BG_OK;
 }
 
 // 2-D map of a row-major bf16 matrix [rows][ld] over its first `cols`
@@ -305,14 +325,10 @@ bool tile_map(CUtensorMap *m, const bf16 *base, int rows, int cols, int ld, int 
 }
 
 template <int NT, bool TMA>
-int launch_gemm_as(const umma::GemmArgs &g, int splits, cudaStream_t st, const CUtensorMap &ta,
+int launch_gemm_as(const umma::GemmArgs &g, int splits, const Device &dev, cudaStream_t st, const CUtensorMap &ta,
                    const CUtensorMap &tb) {
-    static bool attr_set = false;
     constexpr size_t smem = umma::smem_bytes<NT>();
-    if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_gemm<NT, TMA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    if (int rc = raise_smem(dev.id, (const void *)(umma::k_gemm<NT, TMA>), smem)) return rc;
     dim3 grid((unsigned)((g.M + umma::kM - 1) / umma::kM), (unsigned)((g.N + NT - 1) / NT), (unsigned)splits);
     umma::k_gemm<NT, TMA><<<grid, umma::kThreads, smem, st>>>(g, ta, tb);
     MCK(cudaGetLastError());
@@ -338,25 +354,15 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-int sm_count_mlp() {
-    static int n = 0;
-    if (!n) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); if (n <= 0) n = 148; }
-    return n;
-}
-
 // The persistent warp-specialised kernel over all tiles of the product.
 template <int NT>
-int launch_gemm_persistent(const umma::GemmArgs &g, int splits, cudaStream_t st, const CUtensorMap &ta,
+int launch_gemm_persistent(const umma::GemmArgs &g, int splits, const Device &dev, cudaStream_t st, const CUtensorMap &ta,
                            const CUtensorMap &tb) {
-    static bool attr_set = false;
     constexpr size_t smem = umma::psmem_bytes<NT>();
-    if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_gemm_p<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
+    if (int rc = raise_smem(dev.id, (const void *)umma::k_gemm_p<NT>, smem)) return rc;
     const int tiles_m = (g.M + umma::kM - 1) / umma::kM, tiles_n = (g.N + NT - 1) / NT;
     const int ntiles = tiles_m * tiles_n * splits;
-    const int grid = std::max(1, std::min(ntiles, sm_count_mlp()));
+    const int grid = std::max(1, std::min(ntiles, dev.sms));
     MCK(launch_pdl(umma::k_gemm_p<NT>, dim3(grid), dim3(umma::kPThreads), smem, st, g, ta, tb, tiles_m, tiles_n,
                    splits));
     return BG_OK;
@@ -366,39 +372,31 @@ int launch_gemm_persistent(const umma::GemmArgs &g, int splits, cudaStream_t st,
 // aligned rows, K a multiple of 8) and every split has K-chunks, else the
 // one-tile-per-CTA kernel with cp.async stages.
 template <int NT>
-int launch_gemm(const umma::GemmArgs &g, int splits, cudaStream_t st) {
+int launch_gemm(const umma::GemmArgs &g, int splits, const Device &dev, cudaStream_t st) {
     CUtensorMap ta, tb;
     memset(&ta, 0, sizeof ta);
     memset(&tb, 0, sizeof tb);
     if (g.k_per_split >= umma::kKc && g.k_per_split % umma::kKc == 0 && (long long)g.k_per_split * splits == g.K &&
         tile_map(&ta, g.A, g.M, g.K, g.lda, umma::kM, true) && tile_map(&tb, g.B, g.N, g.K, g.ldb, NT, true))
-        return launch_gemm_persistent<NT>(g, splits, st, ta, tb);
+        return launch_gemm_persistent<NT>(g, splits, dev, st, ta, tb);
     memset(&ta, 0, sizeof ta);
     memset(&tb, 0, sizeof tb);
-    return launch_gemm_as<NT, false>(g, splits, st, ta, tb);
+    return launch_gemm_as<NT, false>(g, splits, dev, st, ta, tb);
 }
 
 template <bool BWD>
-int launch_chain(const umma::ChainArgs &g, const umma::ChainMaps &m, cudaStream_t st) {
-    static bool attr_set = false;
+int launch_chain(const umma::ChainArgs &g, const umma::ChainMaps &m, const Device &dev, cudaStream_t st) {
     constexpr size_t smem = umma::chain_smem_bytes();
-    if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_mlp_chain<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
-    const int grid = std::max(1, std::min(g.rows / umma::kM, sm_count_mlp()));
+    if (int rc = raise_smem(dev.id, (const void *)umma::k_mlp_chain<BWD>, smem)) return rc;
+    const int grid = std::max(1, std::min(g.rows / umma::kM, dev.sms));
     MCK(launch_pdl(umma::k_mlp_chain<BWD>, dim3(grid), dim3(umma::kPThreads), smem, st, g, m));
     return BG_OK;
 }
 
-int launch_weight_gradients(const umma::DwArgs &g, const umma::DwMaps &m, cudaStream_t st) {
-    static bool attr_set = false;
+int launch_weight_gradients(const umma::DwArgs &g, const umma::DwMaps &m, const Device &dev, cudaStream_t st) {
     constexpr size_t smem = sizeof(umma::DwSmem);
-    if (!attr_set) {
-        MCK(cudaFuncSetAttribute(umma::k_weight_gradients, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set = true;
-    }
-    const int grid = std::max(1, std::min(g.units, sm_count_mlp()));
+    if (int rc = raise_smem(dev.id, (const void *)umma::k_weight_gradients, smem)) return rc;
+    const int grid = std::max(1, std::min(g.units, dev.sms));
     MCK(launch_pdl(umma::k_weight_gradients, dim3(grid), dim3(umma::kPThreads), smem, st, g, m));
     return BG_OK;
 }
@@ -437,6 +435,7 @@ int dalloc(T **p, size_t n) {
 
 struct bg_mlp {
     int device = 0;
+    Device dev = {0, 148};
     int ydim = 5;
     cudaStream_t stream = nullptr;
     int *err = nullptr;
@@ -597,7 +596,7 @@ int forward(bg_mlp *h, bool keep) {
     umma::ChainArgs g = h->fwd;
     if (!keep)
         for (int l = 0; l < 3; ++l) { g.L[l].keep = 0; g.L[l].mask = nullptr; }
-    return launch_chain<false>(g, h->fwd_maps, h->stream);
+    return launch_chain<false>(g, h->fwd_maps, h->dev, h->stream);
 }
 
 // backward from the loss gradient in h->dO: the hidden layers' gradients -> h->G
@@ -605,14 +604,14 @@ int forward(bg_mlp *h, bool keep) {
 // partial slices -> h->gWl and the bias gradients -> h->gbias.  `advance`: also
 // count the training step.
 int backward(bg_mlp *h, bool advance) {
-    int rc = launch_chain<true>(h->bwd, h->bwd_maps, h->stream);
+    int rc = launch_chain<true>(h->bwd, h->bwd_maps, h->dev, h->stream);
     if (rc) return rc;
     umma::DwArgs g = h->dw;
     if (advance) {
         g.batch_index = (long long *)h->dBatchIdx;
         g.opt_step = (long long *)h->dOptStep;
     }
-    return launch_weight_gradients(g, h->dw_maps, h->stream);
+    return launch_weight_gradients(g, h->dw_maps, h->dev, h->stream);
 }
 
 // Adam's tensor descriptors: gradients from the partial slices of a batch
@@ -717,6 +716,7 @@ BG_API int bg_mlp_create(bg_mlp **out, int device, int ydim) {
     MCK(cudaSetDevice(device));
     bg_mlp *h = new bg_mlp();
     h->device = device;
+    h->dev = device_of(device);
     h->ydim = ydim;
     int rc = 0;
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) rc = fail(BG_ECUDA, "mlp: stream");
@@ -1012,7 +1012,8 @@ BG_API int bg_mlp_gradients(bg_mlp *h, int batch, float *loss, float *const *dW,
 }
 
 // Plain GEMM on device buffers: C[M][N] = A[M][K] . B[N][K]^T (bf16 in,
-// fp32 out), K a multiple of 64; the tensor-core kernel of the network.
+// fp32 out), K a multiple of 64.  k_gemm_p (or k_gemm where no tensor map is
+// allowed) serves this entry point alone: the network's layers are chains.
 BG_API int bg_gemm_bf16(int64_t M, int64_t N, int64_t K, const void *A, const void *B, float *C, void *stream) {
     if (M <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || !A || !B || !C) return fail(BG_EINVAL, "gemm: bad shape");
     // the error flag of the tensor-core waits: one per device, kept for the process
@@ -1027,7 +1028,7 @@ BG_API int bg_gemm_bf16(int64_t M, int64_t N, int64_t K, const void *A, const vo
     umma::GemmArgs g = gemm_args((const bf16 *)A, (int)K, (const bf16 *)B, (int)K, (int)M, (int)N, (int)K, err);
     g.C = C;
     g.ldc = (int)N;
-    int rc = launch_gemm<128>(g, 1, st);
+    int rc = launch_gemm<128>(g, 1, device_of(dev), st);
     cudaError_t e = cudaStreamSynchronize(st);
     int ev = 0;
     cudaMemcpy(&ev, err, sizeof(int), cudaMemcpyDeviceToHost);
