@@ -761,7 +761,7 @@ BG_API int bg_mlp_destroy(bg_mlp *h) {
     for (int l = 0; l < 3; ++l) { dfree(h->H[l]); dfree(h->G[l]); dfree(h->mask[l]); }
     dfree(h->X); dfree(h->dO); dfree(h->OUT); dfree(h->Y); dfree(h->idx);
     for (int l = 0; l < kNLayer; ++l) dfree(h->cs[l]);
-    dfree(h->gW); dfree(h->gflat); dfree(h->loss); dfree(h->Xall); dfree(h->Yall);
+    dfree(h->gW); dfree(h->gbias); dfree(h->gflat); dfree(h->loss); dfree(h->Xall); dfree(h->Yall);
     dfree(h->dBatchIdx); dfree(h->dOptStep); dfree(h->pkeys); dfree(h->pkeys_out); dfree(h->pvals); dfree(h->perm);
     if (h->sort_tmp) cudaFree(h->sort_tmp);
     if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
