@@ -58,8 +58,8 @@ template <typename T> struct StdpStepArgs {
 // placed in a double are w * 2^-896 exactly (zeros and subnormals too), so one
 // FMA gives w + add with the one rounding of the double sum, where widening w
 // takes a conversion on a pipe a quarter as wide as the FP64 one; the clip is a
-// minimum and a maximum.  Both hold for lazy_plain_weight and lazy_plain_add
-// only:
+// minimum and a maximum.  Both hold for weights in [+0, 2^120) and
+// lazy_plain_add only:
 //  - a weight with its sign bit set (-0 among them), infinite or NaN is another
 //    number in that place;
 //  - a NaN sum would leave a minimum and maximum as a bound, where the
@@ -79,7 +79,6 @@ __device__ __forceinline__ WT lazy_update(WT w, double add, float flo, float fhi
         return stdp_w_val<WT>(w, add, wmin, wmax, mode, wx);
     }
 }
-__device__ __forceinline__ bool lazy_plain_weight(float w) { return __float_as_uint(w) < 0x7b800000u; }   // +0 <= w < 2^120
 __device__ __forceinline__ bool lazy_plain_add(double add) {
     const double m = fabs(add);
     return m <= 0x1p100 && !(__double2hiint(add) < 0 && m <= 0x1p-96);
@@ -215,13 +214,14 @@ struct StdpFlushArgs {
 // Applies every pending update to the whole matrix.  A block takes bands of
 // kFlushRows rows: their trace records go to shared memory, with -0 for the
 // steps a row has taken already (w + -0 is w, and such a row was clipped by its
-// presynaptic update since; the general form skips them), then a thread takes
-// one column of the band at a time and walks the column's spikes, all rows of
-// the band side by side.  Warps whose 32 columns have no spikes skip them.
+// presynaptic update since; the instance for the other rules skips them), then a
+// thread takes one column of the band at a time and walks the column's spikes,
+// all rows of the band side by side.  Warps whose 32 columns have no spikes skip
+// them.
 template <typename WT, bool FAST>
 __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArgs a) {
     __shared__ double tab[kFlushRows][kLazySteps];
-    __shared__ int from[kFlushRows];               // first step a row has not taken
+    __shared__ int from[kFlushRows];               // first step a row has not taken (not FAST)
     const int tid = threadIdx.x;
     const int n = (int)(a.ctl->nstep - a.lz->base), win = a.lz->win;
     const unsigned long long *rowmask = a.rowmask + (int64_t)win * a.sn, *colmask = a.colmask + (int64_t)win * a.tn;
@@ -239,13 +239,12 @@ __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArg
         int fits = 1;                              // the band's additions keep the fast form exact
         for (int k = tid; k < kFlushRows * kLazySteps; k += kFlushThreads) {
             const int r = k / kLazySteps, s = k % kLazySteps;
-            const unsigned long long rm = r < rows ? rowmask[i0 + r] : 0ull;
-            const int lo = r >= rows ? kLazySteps : (rm ? 63 - __clzll((long long)rm) : 0);
-            if (s == 0) from[r] = lo;
             double x = -0.0;
-            if (s >= lo && s < n) {
-                x = a.rec[(i0 + r) * kLazySteps + s];
-                fits &= FAST && lazy_plain_add(x);
+            if (r < rows && s < n) {
+                const unsigned long long rm = rowmask[i0 + r];
+                const int lo = rm ? 63 - __clzll((long long)rm) : 0;
+                if (!FAST && s == 0) from[r] = lo;
+                if (s >= lo) { x = a.rec[(i0 + r) * kLazySteps + s]; fits &= lazy_plain_add(x); }
             }
             tab[r][s] = x;
         }
@@ -257,12 +256,14 @@ __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArg
             if (!m) continue;
             WT w[kFlushRows];
             bool plain = FAST && band;
+            int signs = 0;                         // (one unsigned comparison a row made a pass after one step 13 us longer)
 #pragma unroll
             for (int r = 0; r < kFlushRows; ++r) {
                 w[r] = r < rows ? W[(i0 + r) * a.tn + j] : WT(0);
-                plain = plain && lazy_plain_weight((float)w[r]);
+                plain = plain && w[r] < WT(0x1p120);
+                signs |= __float_as_int((float)w[r]);
             }
-            if (plain) {
+            if (plain && signs >= 0) {
                 do {
                     const int s = __ffsll((long long)m) - 1;
                     m &= m - 1;
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kFlushThreads) k_stdp_flush(const StdpFlushArg
                     m &= m - 1;
 #pragma unroll
                     for (int r = 0; r < kFlushRows; ++r)
-                        if (s >= from[r]) w[r] = lazy_update<WT, false>(w[r], tab[r][s], flo, fhi, a.wmin, a.wmax, a.mode, a.wx);
+                        if (FAST || s >= from[r]) w[r] = lazy_update<WT, false>(w[r], tab[r][s], flo, fhi, a.wmin, a.wmax, a.mode, a.wx);
                 } while (m);
             }
 #pragma unroll
