@@ -514,6 +514,14 @@ def profile_case(case, seed):
         d["net"].run(300 * DT)
         sp, _ = d["net"]._binding.rt.counters(2, 1)
         print(json.dumps({"case": "stdp", "steps": 300, "input_spikes": int(sp[0]), "output_spikes": int(sp[1])}))
+    elif case == "cluster":
+        # one CUBA-4000 network, 1000 steps in one launch of k_cluster (its
+        # spike monitor's records are taken after it)
+        from brian_b200 import workloads
+        net = workloads.cuba4000(seed=seed)[0]
+        net.run(1000 * DT)
+        st = net.stats()
+        print(json.dumps({"case": "cluster", "us_per_step": st["last_run_ms"], "blocks": st["cluster_blocks"], "npt": st["cluster_npt"]}))
     elif case == "batch":
         import brian_b200 as b
         from brian_b200 import workloads
@@ -884,11 +892,11 @@ def stdp_bench(args):
             pre_per_step = (int(sp2[0]) - int(sp1[0])) / 200.0
             # algorithmic bytes of the postsynaptic updates: each weight of a
             # spiking column read and written (8 B).  They are applied when a
-            # presynaptic spike needs the weight, or by the flush every 64
+            # presynaptic spike needs the weight, or by the flush every 32
             # steps, so the time set against them is the whole step's
             us = dev_ms * 1e3 / steps
             alg = post_per_step * nin * 8
-            moved = pre_per_step * nout * 8 + nin * nout * 8 / 64
+            moved = pre_per_step * nout * 8 + nin * nout * 8 / 32
             out["kernels_us"] = {k: round(v * 1e3, 3) for k, v in prof}
             out["post_sweep"] = {"kernel": "k_stdp_step and k_stdp_flush (whole step)", "us": us,
                                  "output_spikes_per_step": post_per_step,
@@ -975,7 +983,7 @@ def main():
     ap.add_argument("--fit-batch", type=int, default=16384, help="rows per training step of the proposal network")
     ap.add_argument("--fit-lr", type=float, default=2e-3)
     ap.add_argument("--fit-iters", type=int, default=40)
-    ap.add_argument("--profile-case", choices=["fit", "gemm", "synapses", "synapses_262k", "synapses_262k_stepped", "stdp", "batch"], default=None,
+    ap.add_argument("--profile-case", choices=["fit", "gemm", "synapses", "synapses_262k", "synapses_262k_stepped", "stdp", "batch", "cluster"], default=None,
                     help="run one small case for a single-kernel ncu capture and exit")
     args = ap.parse_args()
     if args.profile_case:

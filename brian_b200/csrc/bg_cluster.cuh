@@ -49,7 +49,8 @@
 // to 50 steps (4000 / 10007 / 16384): 0.88 / 1.16 / 1.21; the persistent
 // kernel, whose chain goes through L2 four times and a polled counter: 2.64 /
 // 3.17 / 3.43 / 3.35 and 2.24 / 2.32 / 2.28.  4000 neurons of a generated
-// conductance model: 1.24, on the stepped launches 14.
+// conductance model: 1.24, on the stepped launches 14.  (The waits' time limit,
+// since then, costs up to 1 % of a step.)
 #pragma once
 #include "bg_kernels.cuh"
 

@@ -109,7 +109,8 @@ struct DevCtl {
 #define BG_DERR_TIMEOUT 3      // a bounded inter-block wait gave up
 #define BG_DERR_NONFINITE 4    // a state variable is NaN or infinite (finite-state check)
 
-// Spin limit of inter-block waits: about a second of polling.
+// Spin limit of inter-block waits: polls (a few seconds of them), in the cluster
+// kernel microseconds too.
 #define BG_SPIN_LIMIT (1u << 22)
 
 __device__ __forceinline__ void bg_finish_step(DevCtl *ctl, int last) {

@@ -305,7 +305,8 @@ struct bg_net {
     // step launches [side0, side1) (the SpikeMonitors, right after the group
     // kernels) only read the spike history the group kernels wrote: in the
     // step graph they run on a side stream beside the launches after them
-    // and join before the step's last launch (the one that advances the step)
+    // and join before the next step's first launch (its group kernels overwrite
+    // what they read; nstep as they need it is kept in DevCtl::mon_step)
     size_t side0 = 0, side1 = 0;
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -9,5 +9,5 @@
 int bg_nvrtc_compile(const std::string &src, std::vector<char> *cubin, std::string *log);
 
 // Kernel sources the network engine compiles with a generated model
-// (bg_common.cuh and bg_kernels.cuh, embedded at build time), in pieces.
+// (build.py's RTC_HEADERS, embedded at build time), in pieces.
 extern const char *const kNetRtcSource[];

@@ -10,7 +10,8 @@
 // -- the same additions, in the same order, each rounded and clipped -- before
 // it is propagated; and every 32 steps, and at the end of a run, one pass
 // over the matrix applies what is pending everywhere (k_stdp_flush).  Results
-// are those of updating every step, bit for bit.
+// are those of updating every step, bit for bit (the sign of a zero and special
+// values included: lazy_update).
 //
 // Updating every step moved the whole matrix each way every step once about
 // half of the targets spike (10 000 x 4096: 328 MB, 52.7 us, at 0.95 of the
@@ -18,7 +19,7 @@
 // 32 steps moves it once; it is bound by the updates' arithmetic (20 M a step:
 // an integer pipe at 0.76 and the conversion pipe at 0.37 of their peaks at
 // 303 us a pass, before the clip became a minimum and a maximum and the sign
-// was taken out: 400 -> 303 -> about 215 us).  A step of that network takes
+// was taken out: 400 -> 303 -> 203 us).  A step of that network takes
 // 26 us, of which the pass is a quarter and the three launches' latency the
 // rest; 2000 x 1000: 23 -> 18 us, 1000 x 64: 19 -> 16 us.
 //

@@ -318,7 +318,9 @@ __device__ __forceinline__ void synp_bins(const SynPersistArgs &a, long long t, 
         }
     }
     __syncthreads();                     // every thread has read the count; shared memory free
-    if (tid == 0) { *cnt = 0; over = 0; }    // (the slot is pushed into again in A(t+3))
+    // the slot takes pushes again in A(t+2) (delay dmax): the clear must stay before
+    // this block's arrival of step t+1, which A(t+2) of every block has waited for
+    if (tid == 0) { *cnt = 0; over = 0; }
 }
 
 template <int NV, bool DIAG>
